@@ -50,18 +50,34 @@ enum : uint32_t { kFlagOverflow = 1, kFlagTimeout = 2, kFlagCapacity = 4, kFlagL
 constexpr uint32_t kStopFlags = kFlagOverflow | kFlagTimeout | kFlagLimit;
 enum : int {
     kCtrTask = 0, kCtrCount = 1, kCtrFlags = 2, kCtrRows = 3, kCtrInter = 4, kCtrElems = 5,
-    kCtrHead = 6, kCtrTail = 7, kCtrActive = 8, kCtrIdle = 9, kCtrDonated = 10, kCtrTailLane = 11,
-    kCtrTailWarp = 12, kCtrIdleNs = 13, kCtrN = 16
+    kCtrTailLane = 6, kCtrTailWarp = 7, kCtrIdleNs = 8, kCtrRead = 16,
+    // cache lines of their own: the number of working warps, the end flag, the idle warps' bitmap
+    kCtrActive = 16, kCtrDone = 32, kCtrIdle = 48, kCtrN = 48 + 256
 };
-// Work-donation ring (a bounded multi-producer multi-consumer queue with a
-// sequence number per slot): a record is [query, level s, lo, hi, idx[0..s-1]].
-constexpr uint32_t kRecWords = 4 + 32;
-constexpr uint64_t kQueueCap = 1u << 16;      // power of two
-// An idle warp polls the ring until no warp is working, a stop flag is set or
-// the run's deadline passes; without a deadline it leaves after kIdleMaxNs
+// Work donation by direct handoff: an idle warp sets its bit in the idle
+// bitmap and polls its own mailbox; a busy warp that sees idle warps clears
+// one warp's bit (which claims that warp) and writes a record
+// [flag, query, level s, lo, hi, idx[0..s-1]] into its mailbox.  Polls touch
+// only the poller's own line.  (A shared ring that every idle warp polled put
+// thousands of polls a microsecond on the line its head, tail and counters
+// share, and every handoff's atomics queued behind them: with chunk survivors
+// donated through it, the 64-query batch of 6 to 8 vertices on 3,112 vertices
+// took 44 ms instead of 30.)
+constexpr uint32_t kMailWords = 64;
+constexpr uint32_t kMaxWarps = 16384;         // bits of the idle bitmap
+enum : uint32_t { kMailEmpty = 0, kMailRecord = 1, kMailDone = 2 };
+static_assert((kCtrN - kCtrIdle) * 64 >= kMaxWarps && kMailWords >= 5 + 32, "donation layout");
+// An idle warp polls until it is handed a record, no warp is working any more
+// or the run's deadline passes; without a deadline it leaves after kIdleMaxNs
 // (the working warps then finish their own ranges, so no work is lost).
 constexpr uint64_t kIdleMaxNs = 3600ull * 1000000000ull;
-constexpr uint32_t kIdleSleepMaxNs = 2048;   // poll back-off ceiling
+constexpr uint64_t kHandoffNs = 1000000000ull;  // longest wait for a record once claimed
+constexpr uint32_t kIdleSleepMaxNs = 512;       // poll back-off ceiling
+// A busy warp looks for idle warps every kDonateEvery steps of its search (a
+// step opens a node or fills a chunk: 1-2 thousand cycles), at the number of
+// working warps it requested at the previous look, so the look waits for no
+// load; flags, time and counts are handled every kCheckEvery steps.
+constexpr uint32_t kDonateEvery = 8, kCheckEvery = 64;
 
 struct DLevel {
     const uint32_t *cand;  // C(u)
@@ -98,8 +114,7 @@ struct EnumArgs {
     unsigned long long count_limit;  // 0 = none
     uint32_t lane_leaf_max;     // longest shortest-list a lane evaluates alone at the last level
     uint32_t merge_ratio;       // a list probe merges (instead of galloping) up to this length ratio
-    uint32_t *queue;            // kQueueCap records of kRecWords words
-    unsigned long long *qseq;   // kQueueCap slot sequence numbers
+    uint32_t *mail;             // a mailbox of kMailWords words per warp of the grid
     // batches of queries (enum_batch_kernel): one QDesc per query, root tasks
     // of query q are task_pre[q] .. task_pre[q+1]
     const struct QDesc *qd;
@@ -217,6 +232,9 @@ struct Warp {
     unsigned long long *local;  // |Vg| x n local counts of the current query (MODE_LOCAL)
     unsigned long long count = 0, inter = 0, elems = 0, tails_lane = 0, tails_warp = 0;
     bool overflow = false;
+    uint32_t wid, nwarps;  // this warp's number in the grid, the grid's warps
+    unsigned long long working = ~0ull;  // working warps as of the last look
+    uint64_t idle_ns = 0;  // lane 0: time spent waiting for work
     uint64_t t_mark = 0;   // lane 0: when this warp's time was last charged to its query
     const unsigned long long *ps;        // kTailChain: prefix sums over the driver edge of level n-2
     const uint32_t *rev_off, *rev_list;  // kTailChain: candidate edges last level -> level n-2
@@ -232,7 +250,8 @@ struct Warp {
     __device__ Warp(const EnumArgs &args, const DLevel *l, const DBack *b, const uint32_t *cf, uint32_t *w, uint32_t ln,
                     uint32_t levels, uint32_t maxn, uint32_t maxnb)
         : a(args), L(l), B(b), CF(cf), lane(ln), n(levels), local(args.local), ps(args.ps), rev_off(args.rev_off),
-          rev_list(args.rev_list), tail(args.tail), xmap_a(args.xmap_a), xmap_z(args.xmap_z), lw(args.lw) {
+          rev_list(args.rev_list), tail(args.tail), xmap_a(args.xmap_a), xmap_z(args.xmap_z), lw(args.lw),
+          wid(blockIdx.x * kWarps + (threadIdx.x >> 5)), nwarps(gridDim.x * kWarps) {
         idx = w;
         vid = idx + maxn;
         buf = vid + maxn;
@@ -865,91 +884,154 @@ struct Warp {
         return key;
     }
 
-    // Gives the upper half of the undispatched driver range of the shallowest
-    // open level to the donation ring (called when more warps are idle than
-    // records are waiting).
-    __device__ void try_donate(uint32_t base, uint32_t d) {
-        uint32_t s = kNone;
-        for (uint32_t l = base; l <= d; ++l)
-            if (dend[l] > dpos[l]) { s = l; break; }
-        if (s == kNone) return;
-        unsigned long long pos = ~0ull;
-        if (lane == 0) {
-            volatile unsigned long long *vc = (volatile unsigned long long *)a.ctr;
-            unsigned long long p = vc[kCtrTail];
-            for (int tries = 0; tries < 64; ++tries) {
-                const unsigned long long seq = *(volatile unsigned long long *)&a.qseq[p & (kQueueCap - 1)];
-                if (seq == p) {
-                    const unsigned long long prev = atomicCAS(&a.ctr[kCtrTail], p, p + 1);
-                    if (prev == p) { pos = p; break; }
-                    p = prev;
-                } else if (seq < p) {
-                    break;  // ring full
-                } else {
-                    p = vc[kCtrTail];
+    // Whether survivors waiting in level l's stack slot may be given away: not
+    // where filling the slot already counted some entries of the chunk lane by
+    // lane (the receiver fills the range anew), nor one level above the last.
+    __device__ __forceinline__ bool slot_donatable(uint32_t l) const {
+        return l + 3 <= n && !(l + 3 == n && lane_tail_ok(l));
+    }
+
+    // The bitmap of idle warps, and one warp claimed from it (kNone when there is none).
+    __device__ __forceinline__ uint32_t *idle_bits() const { return reinterpret_cast<uint32_t *>(a.ctr + kCtrIdle); }
+    __device__ uint32_t claim_idle() {
+        const uint32_t nw = (nwarps + 31) >> 5, start = wid % nw;  // donors start at different words
+        uint32_t *bits = idle_bits();
+        for (uint32_t i0 = 0; i0 < nw; i0 += 32) {
+            const uint32_t i = i0 + lane;
+            uint32_t w = start + i, m = 0;
+            if (w >= nw) w -= nw;
+            if (i < nw) m = *(volatile uint32_t *)(bits + w);
+            uint32_t have = __ballot_sync(kFull, m != 0);
+            while (have) {
+                const int src = __ffs(have) - 1;
+                uint32_t t = kNone;
+                if ((int)lane == src) {
+                    const uint32_t bit = m & (0u - m);
+                    if (atomicAnd(bits + w, ~bit) & bit) t = w * 32 + __ffs(bit) - 1;
                 }
+                t = __shfl_sync(kFull, t, src);
+                if (t != kNone) return t;
+                have &= have - 1;
             }
         }
-        pos = __shfl_sync(kFull, pos, 0);
-        if (pos == ~0ull) return;
-        const uint32_t lo = dpos[s] + (dend[s] - dpos[s]) / 2, hi = dend[s];
-        uint32_t *rec = a.queue + (pos & (kQueueCap - 1)) * kRecWords;
-        if (lane < s) rec[4 + lane] = idx[lane];
+        return kNone;
+    }
+
+    // Hands the upper half of what is left at the shallowest open level to an
+    // idle warp: undispatched driver entries [dpos, dend), and survivors of
+    // the last filled chunk that wait in the level's slot.  Lists are mostly
+    // shorter than one chunk, so without the slots a warp has nothing to give.
+    __device__ void try_donate(uint32_t base, uint32_t d) {
+        uint32_t s = kNone, keep = 0;  // keep: survivors in the slot that stay here
+        bool slot = false;
+        for (uint32_t l = base; l <= d; ++l) {
+            const uint32_t rest = cnt[l] - pos[l], range = dend[l] > dpos[l] ? dend[l] - dpos[l] : 0u;
+            if (!range && !rest) continue;
+            // at the level in work one survivor at least stays; above it the
+            // subtree in work does
+            if (rest > range && slot_donatable(l) && rest >= (l == d ? 2u : 1u)) {
+                s = l;
+                slot = true;
+                keep = rest / 2;
+                break;
+            }
+            if (range) { s = l; break; }
+        }
+        if (s == kNone) return;
+        uint32_t lo = 0, hi = dend[s];
+        if (slot) {
+            // the range starts behind the last survivor kept (or in work): its
+            // place in the driver chunk last filled, [dpos - 32, dpos)
+            const uint32_t p0 = dpos[s] - 32, last = pos[s] + keep;
+            const uint32_t dslot = L[s].back_first + drv[s];
+            lo = p0;
+            if (last) {
+                const uint32_t x = buf[32 * s + last - 1];
+                const uint32_t p = p0 + lane;
+                const uint32_t m = __ballot_sync(kFull, p < hi && B[dslot].list[sstart[dslot] + p] == x);
+                lo = p0 + __ffs(m);  // m has one bit: list entries ascend
+            }
+        } else {
+            lo = dpos[s] + (dend[s] - dpos[s]) / 2;
+        }
+        const uint32_t to = claim_idle();
+        if (to == kNone) return;
+        uint32_t *rec = a.mail + (uint64_t)to * kMailWords;
+        if (lane < s) rec[5 + lane] = idx[lane];
         if (lane == 0) {
-            rec[0] = q;
-            rec[1] = s;
-            rec[2] = lo;
-            rec[3] = hi;
+            rec[1] = q;
+            rec[2] = s;
+            rec[3] = lo;
+            rec[4] = hi;
+            atomicAdd(&a.ctr[kCtrActive], 1ull);  // the receiver's, while this warp still counts
         }
         __threadfence();
         __syncwarp();
         if (lane == 0) {
-            atomicExch(&a.qseq[pos & (kQueueCap - 1)], pos + 1);
-            atomicAdd(&a.ctr[kCtrDonated], 1ull);
+            atomicExch(rec, kMailRecord);
+            if (slot) cnt[s] = pos[s] + keep;
             dend[s] = lo;
         }
         __syncwarp();
     }
 
-    // Idle: polls the donation ring.  Returns the claimed position, or ~0
-    // when no warp is working any more, a stop flag is set, or the wait's
-    // time bound (the run's deadline, else kIdleMaxNs) has passed.  The
-    // caller copies the record and then calls release().
-    __device__ unsigned long long take_queued(uint64_t deadline) {
-        unsigned long long pos = ~0ull;
+    // This warp stops working; the last one to stop ends the run for the
+    // waiting warps.
+    __device__ void leave_active() {
+        bool last = false;
         if (lane == 0) {
-            volatile unsigned long long *vc = (volatile unsigned long long *)a.ctr;
-            atomicAdd(&a.ctr[kCtrIdle], 1ull);
-            const uint64_t t0 = globaltimer();
-            const uint64_t until = deadline ? deadline : t0 + kIdleMaxNs;
-            uint32_t nap = 128;
-            for (uint32_t it = 0;; ++it) {
-                const unsigned long long p = vc[kCtrHead];
-                const unsigned long long seq = *(volatile unsigned long long *)&a.qseq[p & (kQueueCap - 1)];
-                if (seq == p + 1) {
-                    if (atomicCAS(&a.ctr[kCtrHead], p, p + 1) == p) { pos = p; break; }
-                    nap = 128;
-                } else if (seq < p + 1) {
-                    if (vc[kCtrActive] == 0 || (vc[kCtrFlags] & kStopFlags)) break;
-                    if ((it & 255u) == 255u && globaltimer() > until) break;
-                    __nanosleep(nap);
-                    nap = min(2 * nap, kIdleSleepMaxNs);
-                }
-            }
-            if (pos != ~0ull) atomicAdd(&a.ctr[kCtrActive], 1ull);
-            atomicAdd(&a.ctr[kCtrIdleNs], (unsigned long long)(globaltimer() - t0));
-            atomicAdd(&a.ctr[kCtrIdle], ~0ull);
             __threadfence();
+            last = atomicAdd(&a.ctr[kCtrActive], ~0ull) == 1ull;
+            if (last) {
+                atomicExch(&a.ctr[kCtrDone], 1ull);
+                __threadfence();
+            }
         }
-        return __shfl_sync(kFull, pos, 0);
+        if (__shfl_sync(kFull, last, 0))
+            for (uint32_t w = lane; w < nwarps; w += 32) atomicExch(a.mail + (uint64_t)w * kMailWords, kMailDone);
     }
 
-    __device__ void release(unsigned long long pos) {
-        __syncwarp();
+    // Idle: waits for a record in this warp's mailbox.  False when no warp is
+    // working any more or the wait's time bound (the run's deadline, else
+    // kIdleMaxNs) has passed.
+    __device__ bool wait_work(uint64_t deadline) {
+        bool got = false;
         if (lane == 0) {
+            uint32_t *mb = a.mail + (uint64_t)wid * kMailWords, *word = idle_bits() + (wid >> 5);
+            const uint32_t bit = 1u << (wid & 31u);
+            atomicExch(mb, kMailEmpty);
             __threadfence();
-            atomicExch(&a.qseq[pos & (kQueueCap - 1)], pos + kQueueCap);
+            atomicOr(word, bit);
+            __threadfence();
+            const uint64_t t0 = globaltimer();
+            uint64_t until = deadline ? deadline : t0 + kIdleMaxNs;
+            bool claimed = false;
+            uint32_t nap = 64;
+            // a run that ended before the mailbox was emptied shows in the end flag
+            bool wait = *(volatile unsigned long long *)&a.ctr[kCtrDone] == 0;
+            for (uint32_t it = 0; wait; ++it) {
+                const uint32_t f = *(volatile uint32_t *)mb;
+                if (f != kMailEmpty) {
+                    got = f == kMailRecord;
+                    break;
+                }
+                if ((it & 255u) == 255u && globaltimer() > until) {
+                    if (claimed) {  // a claimed warp's record did not come: cannot happen, not a count to trust
+                        atomicOr((unsigned int *)&a.ctr[kCtrFlags], kFlagTimeout);
+                        break;
+                    }
+                    if (atomicAnd(word, ~bit) & bit) break;
+                    claimed = true;  // a donor took the bit first: its record is on the way
+                    until = globaltimer() + kHandoffNs;
+                }
+                __nanosleep(nap);
+                nap = min(2 * nap, kIdleSleepMaxNs);
+            }
+            idle_ns += globaltimer() - t0;
+            __threadfence();
         }
+        __syncwarp();
+        return __shfl_sync(kFull, got, 0);
     }
 
     // Membership of x (this lane's driver element) in every non-driver list
@@ -1195,8 +1277,14 @@ __device__ bool dfs(const EnumArgs &a, Warp<MODE, MULTI> &W, uint32_t lane, uint
     const uint32_t n = W.n;
     uint32_t d = base;
     while (d >= base) {
-        if ((++iter & 63u) == 0) {
-            uint32_t st = 0, want = 0;
+        ++iter;
+        if ((iter & (kDonateEvery - 1)) == 0) {
+            if (W.working < W.nwarps) W.try_donate(base, d);
+            // one load for the warp, used at the next look
+            asm volatile("ld.volatile.global.u64 %0, [%1];" : "=l"(W.working) : "l"(a.ctr + kCtrActive));
+        }
+        if ((iter & (kCheckEvery - 1)) == 0) {
+            uint32_t st = 0;
             W.flush_count();
             if (lane == 0) {
                 st = *flags & kStopFlags;
@@ -1204,13 +1292,9 @@ __device__ bool dfs(const EnumArgs &a, Warp<MODE, MULTI> &W, uint32_t lane, uint
                     atomicOr((unsigned int *)&a.ctr[kCtrFlags], kFlagTimeout);
                     st = kFlagTimeout;
                 }
-                volatile unsigned long long *vc = (volatile unsigned long long *)a.ctr;
-                const unsigned long long idle = vc[kCtrIdle], pend = vc[kCtrTail] - vc[kCtrHead];
-                want = idle > pend && (long long)pend >= 0;
             }
             if (__shfl_sync(kFull, st, 0)) return false;
             if (W.query_stopped()) return true;  // abandon this query's subtree
-            if (__shfl_sync(kFull, want, 0)) W.try_donate(base, d);
         }
         if (W.pos[d] < W.cnt[d]) {
             const uint32_t x = W.buf[32 * d + W.pos[d]];
@@ -1295,18 +1379,17 @@ template <uint32_t MODE, bool MULTI>
 __device__ void warp_loop(const EnumArgs &a, Warp<MODE, MULTI> &W, uint32_t lane) {
     const unsigned long long nblocks = MULTI ? a.task_pre[a.nquery] : a.ntasks;
     uint32_t iter = 0;
-    bool stop = false, roots_left = true;
+    bool stop = false, roots_left = true, working = true;
     uint64_t deadline = 0;
     if (a.limit_ns && lane == 0) deadline = globaltimer() + a.limit_ns;
-    // a warp counts as active (kCtrActive) from its first root task until the
-    // roots run out, not per task: fewer atomics on one hot counter
+    // a warp counts as working from here until it finds neither a root task
+    // nor, after it, anything left of a record it was handed
     if (lane == 0) atomicAdd(&a.ctr[kCtrActive], 1ull);
     while (!stop) {
         if (roots_left) {
             unsigned long long b = 0;
             if (lane == 0) {
                 b = atomicAdd(&a.ctr[kCtrTask], 1ull);
-                if (b >= nblocks) atomicAdd(&a.ctr[kCtrActive], ~0ull);
             }
             b = __shfl_sync(kFull, b, 0);
             if (b < nblocks) {
@@ -1365,29 +1448,26 @@ __device__ void warp_loop(const EnumArgs &a, Warp<MODE, MULTI> &W, uint32_t lane
             }
             roots_left = false;
         }
-        const unsigned long long qpos = W.take_queued(deadline);
-        if (qpos == ~0ull) break;
-        const volatile uint32_t *rec = a.queue + (qpos & (kQueueCap - 1)) * kRecWords;
-        if (MULTI) W.bind(rec[0]);
-        const uint32_t s = rec[1], lo = rec[2], hi = rec[3];
+        W.leave_active();
+        working = false;
+        if (!W.wait_work(deadline)) break;
+        working = true;  // counted by the donor
+        const volatile uint32_t *rec = a.mail + (uint64_t)W.wid * kMailWords;
+        if (MULTI) W.bind(rec[1]);
+        const uint32_t s = rec[2], lo = rec[3], hi = rec[4];
         if (lane < s) {
-            const uint32_t x = rec[4 + lane];
+            const uint32_t x = rec[5 + lane];
             W.idx[lane] = x;
             W.vid[lane] = W.L[lane].cand[x];
         }
-        W.release(qpos);
         __syncwarp();
         const long long c0 = clock64();
         W.mark();
         if (!W.query_stopped()) stop = !run_range(a, W, lane, s, lo, hi, iter, deadline);
         W.charge();
-        if (lane == 0) {
-            if (MULTI && a.qcycles) atomicAdd(&a.qcycles[W.q], (unsigned long long)(clock64() - c0));
-            atomicAdd(&a.ctr[kCtrActive], ~0ull);
-        }
+        if (lane == 0 && MULTI && a.qcycles) atomicAdd(&a.qcycles[W.q], (unsigned long long)(clock64() - c0));
     }
-    // a warp stopped while it still had roots leaves the active count
-    if (roots_left && lane == 0) atomicAdd(&a.ctr[kCtrActive], ~0ull);
+    if (working) W.leave_active();  // stopped early
     // flush per-warp totals
     W.flush_count();
     if (lane == 0) {
@@ -1395,6 +1475,7 @@ __device__ void warp_loop(const EnumArgs &a, Warp<MODE, MULTI> &W, uint32_t lane
         atomicAdd(&a.ctr[kCtrElems], W.elems);
         atomicAdd(&a.ctr[kCtrTailLane], W.tails_lane);
         atomicAdd(&a.ctr[kCtrTailWarp], W.tails_warp);
+        atomicAdd(&a.ctr[kCtrIdleNs], (unsigned long long)W.idle_ns);
     }
 }
 
@@ -1423,8 +1504,10 @@ __global__ void __launch_bounds__(kThreads) enum_kernel(EnumArgs a) {
 // Many queries in one persistent launch (COUNT mode): root tasks of every
 // query form one range claimed by atomicAdd, plans are read from global
 // memory, counts go to per-query totals.
+// At least two blocks stay resident per SM (128 registers a thread) whatever
+// the tuning asks: at one, half of the warps that hide the loads are gone.
 template <int MINB, uint32_t MODE = ASDM_MODE_COUNT>
-__global__ void __launch_bounds__(kThreads, MINB) enum_batch_kernel(EnumArgs a) {
+__global__ void __launch_bounds__(kThreads, MINB < 2 ? 2 : MINB) enum_batch_kernel(EnumArgs a) {
     extern __shared__ __align__(16) uint32_t sm[];
     const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     uint32_t *wmem = sm + warp * warp_words(a.maxn, a.maxnb);
@@ -1583,11 +1666,6 @@ __global__ void cross_index(const XSeg *__restrict__ seg, uint32_t nseg, unsigne
     }
 }
 
-__global__ void queue_init(unsigned long long *seq) {
-    const uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < kQueueCap) seq[i] = i;
-}
-
 template <uint32_t MODE>
 int launch(const EnumArgs &a, uint32_t smem, int num_sms, cudaStream_t s) {
     auto k = enum_kernel<MODE>;
@@ -1596,7 +1674,7 @@ int launch(const EnumArgs &a, uint32_t smem, int num_sms, cudaStream_t s) {
     ASDM_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, kThreads, smem));
     if (per_sm <= 0) return fail(ASDM_ERR_INVALID, "query too large for one block's shared memory (%u bytes)", smem);
     // persistent grid: warps without a root task steal donated work
-    const unsigned grid = (unsigned)std::max(1, per_sm * num_sms);
+    const unsigned grid = (unsigned)std::max(1, std::min(per_sm * num_sms, (int)kMaxWarps / kWarps));
     k<<<grid, kThreads, smem, s>>>(a);
     ::asdm::count_launch();
     ASDM_CUDA(cudaGetLastError());
@@ -1868,7 +1946,7 @@ int run_plan(asdm_cs &cs, const asdm_plan &plan, const asdm_run_opts &opt, asdm_
     std::memcpy(hp.data() + n * sizeof(DLevel) + nb * sizeof(DBack), cf.data(), nc * sizeof(uint32_t));
     uint8_t *d_plan = nullptr;
     unsigned long long *d_ctr = nullptr, *d_local = nullptr, *d_ps = nullptr;
-    uint32_t *d_rows = nullptr, *d_queue = nullptr, *d_xmap = nullptr;
+    uint32_t *d_rows = nullptr, *d_mail = nullptr, *d_xmap = nullptr;
     unsigned long long *d_lw = nullptr;
     int rc = ASDM_OK;
     auto cleanup = [&]() {
@@ -1879,7 +1957,7 @@ int run_plan(asdm_cs &cs, const asdm_plan &plan, const asdm_run_opts &opt, asdm_
         dfree(d_ctr, s);
         dfree(d_local, s);
         dfree(d_rows, s);
-        dfree(d_queue, s);
+        dfree(d_mail, s);
     };
     EnumArgs a{};
     uint64_t row_cap = 0;
@@ -1887,14 +1965,7 @@ int run_plan(asdm_cs &cs, const asdm_plan &plan, const asdm_run_opts &opt, asdm_
     do {
         if ((rc = dalloc(&d_plan, pbytes, s))) break;
         if ((rc = dalloc(&d_ctr, kCtrN, s))) break;
-        if ((rc = dalloc(&d_queue, kQueueCap * kRecWords + 2 * kQueueCap, s))) break;
-        queue_init<<<(unsigned)(kQueueCap / 256), 256, 0, s>>>(
-            reinterpret_cast<unsigned long long *>(d_queue + kQueueCap * kRecWords));
-        ::asdm::count_launch();
-        if (cudaGetLastError() != cudaSuccess) {
-            rc = fail(ASDM_ERR_CUDA, "queue reset failed");
-            break;
-        }
+        if ((rc = dalloc(&d_mail, (uint64_t)kMaxWarps * kMailWords, s))) break;
         if (cudaMemcpyAsync(d_plan, hp.data(), pbytes, cudaMemcpyHostToDevice, s) != cudaSuccess ||
             cudaMemsetAsync(d_ctr, 0, kCtrN * sizeof(unsigned long long), s) != cudaSuccess) {
             rc = fail(ASDM_ERR_CUDA, "plan upload failed");
@@ -1924,8 +1995,7 @@ int run_plan(asdm_cs &cs, const asdm_plan &plan, const asdm_run_opts &opt, asdm_
         a.local = d_local;
         a.rows = d_rows;
         a.row_cap = row_cap;
-        a.queue = d_queue;
-        a.qseq = reinterpret_cast<unsigned long long *>(d_queue + kQueueCap * kRecWords);
+        a.mail = d_mail;
         a.limit_ns = opt.time_limit_s > 0 ? (uint64_t)(opt.time_limit_s * 1e9) : 0;
         a.count_limit = opt.count_limit;
         a.lane_leaf_max = G->tuning.lane_leaf_max;
@@ -1960,7 +2030,7 @@ int run_plan(asdm_cs &cs, const asdm_plan &plan, const asdm_run_opts &opt, asdm_
             if (rc) break;
         }
         cudaEventRecord(e1, s);
-        unsigned long long ctr[kCtrN];
+        unsigned long long ctr[kCtrRead];
         if (cudaMemcpyAsync(ctr, d_ctr, sizeof ctr, cudaMemcpyDeviceToHost, s) != cudaSuccess) {
             rc = fail(ASDM_ERR_CUDA, "counter readback failed");
             break;
@@ -2266,7 +2336,7 @@ int run_batch_count(asdm_graph *G, const std::vector<asdm_cs *> &cs, const std::
     uint8_t *d_buf = nullptr;
     unsigned long long *d_ctr = nullptr, *d_qcounts = nullptr, *d_local = nullptr, *d_ps = nullptr, *d_cyc = nullptr;
     unsigned long long *d_qwork = nullptr;
-    uint32_t *d_queue = nullptr, *d_xmap = nullptr;
+    uint32_t *d_mail = nullptr, *d_xmap = nullptr;
     unsigned long long *d_lw = nullptr;
     std::vector<unsigned long long *> lwv;
     unsigned int *d_qflags = nullptr;
@@ -2287,7 +2357,7 @@ int run_batch_count(asdm_graph *G, const std::vector<asdm_cs *> &cs, const std::
         }
         if ((rc = dalloc(&d_buf, hp.size(), s)) || (rc = dalloc(&d_ctr, kCtrN, s)) ||
             (rc = dalloc(&d_qcounts, 2ull * L, s)) || (rc = dalloc(&d_qflags, L, s)) ||
-            (rc = dalloc(&d_queue, kQueueCap * kRecWords + 2 * kQueueCap, s)))
+            (rc = dalloc(&d_mail, (uint64_t)kMaxWarps * kMailWords, s)))
             break;
         d_qwork = d_qcounts + L;
         if (!local_mode) {
@@ -2333,13 +2403,9 @@ int run_batch_count(asdm_graph *G, const std::vector<asdm_cs *> &cs, const std::
             rc = fail(ASDM_ERR_CUDA, "batch upload failed");
             break;
         }
-        unsigned long long *d_seq = reinterpret_cast<unsigned long long *>(d_queue + kQueueCap * kRecWords);
-        queue_init<<<(unsigned)(kQueueCap / 256), 256, 0, s>>>(d_seq);
-        ::asdm::count_launch();
         EnumArgs a{};
         a.ctr = d_ctr;
-        a.queue = d_queue;
-        a.qseq = d_seq;
+        a.mail = d_mail;
         a.qd = reinterpret_cast<const QDesc *>(d_buf + qd_at);
         a.task_pre = reinterpret_cast<const unsigned long long *>(d_buf + tp_at);
         a.nquery = L;
@@ -2386,10 +2452,11 @@ int run_batch_count(asdm_graph *G, const std::vector<asdm_cs *> &cs, const std::
                 rc = fail(ASDM_ERR_INVALID, "batch plans too large for shared memory (%u bytes)", smem);
                 break;
             }
+            const int grid = std::min(per_sm * G->num_sms, (int)kMaxWarps / kWarps);
             // a query's budget: its time alone on the GPU, as warp-time over every resident warp
             if (query_time_s > 0)
-                a.q_budget_ns = (unsigned long long)(query_time_s * 1e9 * (double)per_sm * G->num_sms * kWarps);
-            k<<<(unsigned)(per_sm * G->num_sms), kThreads, smem, s>>>(a);
+                a.q_budget_ns = (unsigned long long)(query_time_s * 1e9 * (double)grid * kWarps);
+            k<<<(unsigned)grid, kThreads, smem, s>>>(a);
             ::asdm::count_launch();
             if (cudaGetLastError() != cudaSuccess) {
                 rc = fail(ASDM_ERR_CUDA, "batch kernel launch failed");
@@ -2397,7 +2464,7 @@ int run_batch_count(asdm_graph *G, const std::vector<asdm_cs *> &cs, const std::
             }
         }
         cudaEventRecord(e1, s);
-        unsigned long long ctr[kCtrN];
+        unsigned long long ctr[kCtrRead];
         std::vector<unsigned long long> qc(2ull * L);  // counts, then warp-time charged
         std::vector<unsigned int> qf(L);
         if (cudaMemcpyAsync(ctr, d_ctr, sizeof ctr, cudaMemcpyDeviceToHost, s) != cudaSuccess ||
@@ -2477,7 +2544,7 @@ int run_batch_count(asdm_graph *G, const std::vector<asdm_cs *> &cs, const std::
     dfree(d_ctr, s);
     dfree(d_qcounts, s);
     dfree(d_qflags, s);
-    dfree(d_queue, s);
+    dfree(d_mail, s);
     dfree(d_local, s);
     cudaStreamSynchronize(s);
     return rc;
@@ -2546,28 +2613,27 @@ extern "C" int asdm_cs_count_lower_bound(asdm_cs *cs, uint64_t *lower, int *exce
 // implicit device synchronisation.  asdm_run_plan_count_noalloc serves them:
 // it runs the same COUNT-mode enumeration kernel as asdm_run_plan, but its
 // scratch (the run counters, the device copy of the plan and the
-// work-donation ring) lives in the fixed, file-scope device array below.
+// work-donation mailboxes) lives in the fixed, file-scope device array below.
 // The caller still passes the inputs (a candidate space and a plan) and the
 // output (the stats struct).
 //
-// The array is kNoAllocScratchBytes (about 10 MiB) on every GPU that loads
+// The array is kNoAllocScratchBytes (about 4 MiB) on every GPU that loads
 // this library, held until the process exits.  Its host-side name is only a
 // stand-in for the device symbol, so the device address is fetched with
 // cudaGetSymbolAddress once per device (with that device current) by the
 // first call made on that device; make that first call before any stream
 // capture.  All calls share the one array and it keeps the last call's
-// contents: every call re-zeroes the counters and re-initialises the ring
-// before its launch.  Calls that overlap on the GPU (from several host
+// contents: every call re-zeroes the counters before its launch.  Calls that overlap on the GPU (from several host
 // threads or several streams) race on the array and must be serialised by
 // the caller.
 namespace asdm {
 namespace {
 
-constexpr uint64_t kNoAllocCtrBytes = 256;
+constexpr uint64_t kNoAllocCtrBytes = 4096;
 constexpr uint64_t kNoAllocPlanBytes = 16384;  // >= 32 levels + 496 back edges + 496 conflict levels
-constexpr uint64_t kNoAllocSeqBytes = kQueueCap * sizeof(unsigned long long);
-constexpr uint64_t kNoAllocRingBytes = kQueueCap * kRecWords * sizeof(uint32_t);
-constexpr uint64_t kNoAllocScratchBytes = kNoAllocCtrBytes + kNoAllocPlanBytes + kNoAllocSeqBytes + kNoAllocRingBytes;
+constexpr uint64_t kNoAllocMailBytes = (uint64_t)kMaxWarps * kMailWords * sizeof(uint32_t);
+constexpr uint64_t kNoAllocScratchBytes = kNoAllocCtrBytes + kNoAllocPlanBytes + kNoAllocMailBytes;
+static_assert(kNoAllocCtrBytes >= kCtrN * sizeof(unsigned long long), "no-alloc counters");
 
 static __device__ __align__(256) unsigned char g_noalloc_scratch[kNoAllocScratchBytes];
 
@@ -2639,15 +2705,10 @@ extern "C" int asdm_run_plan_count_noalloc(asdm_cs *cs, const asdm_plan *plan, d
     ASDM_TRY(noalloc_scratch(G->device, &base));
     unsigned long long *d_ctr = reinterpret_cast<unsigned long long *>(base);
     uint8_t *d_plan = base + kNoAllocCtrBytes;
-    unsigned long long *d_seq = reinterpret_cast<unsigned long long *>(base + kNoAllocCtrBytes + kNoAllocPlanBytes);
-    uint32_t *d_ring = reinterpret_cast<uint32_t *>(base + kNoAllocCtrBytes + kNoAllocPlanBytes + kNoAllocSeqBytes);
+    uint32_t *d_mail = reinterpret_cast<uint32_t *>(base + kNoAllocCtrBytes + kNoAllocPlanBytes);
 
     ASDM_CUDA(cudaMemcpyAsync(d_plan, hp.data(), pbytes, cudaMemcpyHostToDevice, s));
     ASDM_CUDA(cudaMemsetAsync(d_ctr, 0, kCtrN * sizeof(unsigned long long), s));
-    queue_init<<<(unsigned)(kQueueCap / 256), 256, 0, s>>>(d_seq);
-    ::asdm::count_launch();
-    ASDM_CUDA(cudaGetLastError());
-
     EnumArgs a{};
     a.lv = reinterpret_cast<const DLevel *>(d_plan);
     a.bk = reinterpret_cast<const DBack *>(d_plan + n * sizeof(DLevel));
@@ -2658,8 +2719,7 @@ extern "C" int asdm_run_plan_count_noalloc(asdm_cs *cs, const asdm_plan *plan, d
     a.nq = n;
     root_blocks(*cs, *plan, a.pairs, a.blk, a.ntasks);
     a.ctr = d_ctr;
-    a.queue = d_ring;
-    a.qseq = d_seq;
+    a.mail = d_mail;
     a.limit_ns = time_limit_s > 0 ? (uint64_t)(time_limit_s * 1e9) : 0;
     a.count_limit = count_limit;
     a.lane_leaf_max = G->tuning.lane_leaf_max;
@@ -2668,7 +2728,7 @@ extern "C" int asdm_run_plan_count_noalloc(asdm_cs *cs, const asdm_plan *plan, d
         const uint32_t smem = 4u * (plan_words(n, nb, nc) + kWarps * warp_words(n, nb));
         ASDM_TRY(launch<ASDM_MODE_COUNT>(a, smem, G->num_sms, s));
     }
-    unsigned long long ctr[kCtrN];
+    unsigned long long ctr[kCtrRead];
     ASDM_CUDA(cudaMemcpyAsync(ctr, d_ctr, sizeof ctr, cudaMemcpyDeviceToHost, s));
     ASDM_CUDA(cudaStreamSynchronize(s));
     stats->count = ctr[kCtrCount];

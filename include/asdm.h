@@ -276,7 +276,7 @@ int asdm_run_plan(asdm_cs *cs, const asdm_plan *plan, const asdm_run_opts *opts,
  * for callers whose GPU memory is fully reserved by their own allocator, or
  * that cannot afford cudaMalloc/cudaFree (and their implicit synchronisation)
  * while they run.  The kernel's scratch (counters, device plan, work-donation
- * ring) is a fixed ~10 MiB file-scope device array, held by every GPU that
+ * mailboxes) is a fixed ~4 MiB file-scope device array, held by every GPU that
  * loads the library until exit.  The first call on a device looks up that
  * array's address (cudaGetSymbolAddress) with the graph's device current, so
  * make it before any stream capture.  Calls share the array and must not
