@@ -112,6 +112,7 @@ struct EnumArgs {
     uint64_t row_cap;
     uint64_t limit_ns;          // 0 = none; else per-warp wall-clock budget
     unsigned long long count_limit;  // 0 = none
+    unsigned long long flush_at;     // a warp adds its count to the total as soon as it is this large (limit_flush)
     uint32_t lane_leaf_max;     // longest shortest-list a lane evaluates alone at the last level
     uint32_t merge_ratio;       // a list probe merges (instead of galloping) up to this length ratio
     uint32_t *mail;             // a mailbox of kMailWords words per warp of the grid
@@ -176,6 +177,15 @@ constexpr uint32_t kLaneTailWork = 64;
 
 __host__ __device__ inline uint32_t plan_words(uint32_t n, uint32_t nb, uint32_t nc) {
     return (uint32_t)((n * sizeof(DLevel) + nb * sizeof(DBack)) / 4) + ((nc + 3) & ~3u);
+}
+
+// With a count limit a warp passes its count on once it reaches a 1,024th of
+// the limit: closed-form tails can add 10^8 matches in one step, so a query
+// would otherwise run on for up to kCheckEvery steps of every warp after its
+// limit (5-vertex queries on 3.77M vertices counted 10^10 matches under a
+// limit of 10^8).
+inline unsigned long long limit_flush(uint64_t count_limit) {
+    return count_limit ? std::max<unsigned long long>(1, count_limit >> 10) : ~0ull;
 }
 
 __device__ __forceinline__ uint64_t globaltimer() {
@@ -1283,7 +1293,7 @@ __device__ bool dfs(const EnumArgs &a, Warp<MODE, MULTI> &W, uint32_t lane, uint
             // one load for the warp, used at the next look
             asm volatile("ld.volatile.global.u64 %0, [%1];" : "=l"(W.working) : "l"(a.ctr + kCtrActive));
         }
-        if ((iter & (kCheckEvery - 1)) == 0) {
+        if ((iter & (kCheckEvery - 1)) == 0 || W.count >= a.flush_at) {
             uint32_t st = 0;
             W.flush_count();
             if (lane == 0) {
@@ -1407,6 +1417,7 @@ __device__ void warp_loop(const EnumArgs &a, Warp<MODE, MULTI> &W, uint32_t lane
                 // a query past its count limit or time budget is abandoned: its remaining
                 // root tasks are skipped at once (the task counter jumps past them)
                 W.mark();
+                if (W.count >= a.flush_at) W.flush_count();
                 if (W.query_stopped()) {
                     t_end = t;
                     if (MULTI && lane == 0) atomicMax(&a.ctr[kCtrTask], a.task_pre[W.q + 1]);
@@ -1998,6 +2009,7 @@ int run_plan(asdm_cs &cs, const asdm_plan &plan, const asdm_run_opts &opt, asdm_
         a.mail = d_mail;
         a.limit_ns = opt.time_limit_s > 0 ? (uint64_t)(opt.time_limit_s * 1e9) : 0;
         a.count_limit = opt.count_limit;
+        a.flush_at = limit_flush(a.count_limit);
         a.lane_leaf_max = G->tuning.lane_leaf_max;
         a.merge_ratio = G->tuning.merge_ratio;
         if (mode == ASDM_MODE_COUNT) {
@@ -2424,6 +2436,7 @@ int run_batch_count(asdm_graph *G, const std::vector<asdm_cs *> &cs, const std::
         }
         a.limit_ns = time_limit_s > 0 ? (uint64_t)(time_limit_s * 1e9) : 0;
         a.count_limit = count_limit;
+        a.flush_at = limit_flush(a.count_limit);
         const uint32_t smem = 4u * kWarps * warp_words(maxn, maxnb);
         cudaEventCreate(&e0);
         cudaEventCreate(&e1);
@@ -2722,6 +2735,7 @@ extern "C" int asdm_run_plan_count_noalloc(asdm_cs *cs, const asdm_plan *plan, d
     a.mail = d_mail;
     a.limit_ns = time_limit_s > 0 ? (uint64_t)(time_limit_s * 1e9) : 0;
     a.count_limit = count_limit;
+    a.flush_at = limit_flush(a.count_limit);
     a.lane_leaf_max = G->tuning.lane_leaf_max;
     a.merge_ratio = G->tuning.merge_ratio;
     if (a.ntasks) {
