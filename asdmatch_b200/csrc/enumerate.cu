@@ -26,9 +26,9 @@
 #include <cstring>
 #include <memory>
 #include <mutex>
-#include <numeric>
 
 #include "cs.cuh"
+#include "rows.cuh"
 
 namespace asdm {
 
@@ -108,8 +108,12 @@ struct EnumArgs {
     unsigned long long blk;     // pairs per root block
     unsigned long long *ctr;
     unsigned long long *local;  // |Vg| x nq, MODE_LOCAL
-    uint32_t *rows;             // row_cap x nq, MODE_EMBED
+    // MODE_EMBED: rows as packed keys (rows.cuh), word k of row r at
+    // rows[k * row_cap + r]; field[u] = word << 8 | shift of query vertex u
+    unsigned long long *rows;
     uint64_t row_cap;
+    const uint32_t *field;
+    uint32_t row_words;
     uint64_t limit_ns;          // 0 = none; else per-warp wall-clock budget
     unsigned long long count_limit;  // 0 = none
     unsigned long long flush_at;     // a warp adds its count to the total as soon as it is this large (limit_flush)
@@ -1174,16 +1178,22 @@ struct Warp {
         __syncwarp();
     }
 
-    __device__ void emit_rows(uint32_t d, uint32_t vx, bool ok, uint32_t mask) {
+    // x: this lane's candidate of level d, the last level of its match.
+    __device__ void emit_rows(uint32_t d, uint32_t x, bool ok, uint32_t mask) {
         unsigned long long base = 0;
         if (lane == 0 && mask) base = atomicAdd(&a.ctr[kCtrRows], (unsigned long long)__popc(mask));
         base = __shfl_sync(kFull, base, 0);
         if (ok) {
             const unsigned long long r = base + __popc(mask & ((1u << lane) - 1));
             if (r < a.row_cap) {
-                uint32_t *row = a.rows + r * n;
-                for (uint32_t j = 0; j < d; ++j) row[L[j].u] = vid[j];
-                row[L[d].u] = vx;
+                for (uint32_t k = 0; k < a.row_words; ++k) {
+                    unsigned long long key = 0;
+                    for (uint32_t j = 0; j <= d; ++j) {
+                        const uint32_t f = a.field[L[j].u];
+                        if ((f >> 8) == k) key |= (unsigned long long)(j == d ? x : idx[j]) << (f & 255u);
+                    }
+                    a.rows[(unsigned long long)k * a.row_cap + r] = key;
+                }
             } else {
                 atomicOr((unsigned int *)&a.ctr[kCtrFlags], kFlagCapacity);
             }
@@ -1256,7 +1266,7 @@ struct Warp {
                 const uint32_t mask = __ballot_sync(kFull, ok);
                 total += __popc(mask);
                 if ((MODE & ASDM_MODE_LOCAL) && ok) atomicAdd(&local[(unsigned long long)vx * n + lv.u], 1ull);
-                if (MODE & ASDM_MODE_EMBED) emit_rows(d, vx, ok, mask);
+                if (MODE & ASDM_MODE_EMBED) emit_rows(d, x, ok, mask);
             }
             if ((MODE & ASDM_MODE_LOCAL) && total && lane < d)
                 atomicAdd(&local[(unsigned long long)vid[lane] * n + L[lane].u], total);
@@ -1271,8 +1281,7 @@ struct Warp {
             if (lane <= d) atomicAdd(&local[(unsigned long long)vid[lane] * n + L[lane].u], 1ull);
         }
         if (MODE & ASDM_MODE_EMBED) {
-            const uint32_t vx = vid[d];
-            emit_rows(d, vx, lane == 0, 1u);
+            emit_rows(d, idx[d], lane == 0, 1u);
         }
     }
 };
@@ -1957,7 +1966,9 @@ int run_plan(asdm_cs &cs, const asdm_plan &plan, const asdm_run_opts &opt, asdm_
     std::memcpy(hp.data() + n * sizeof(DLevel) + nb * sizeof(DBack), cf.data(), nc * sizeof(uint32_t));
     uint8_t *d_plan = nullptr;
     unsigned long long *d_ctr = nullptr, *d_local = nullptr, *d_ps = nullptr;
-    uint32_t *d_rows = nullptr, *d_mail = nullptr, *d_xmap = nullptr;
+    uint32_t *d_mail = nullptr, *d_xmap = nullptr, *d_field = nullptr;
+    unsigned long long *d_rows = nullptr;
+    RowLayout lay;
     unsigned long long *d_lw = nullptr;
     int rc = ASDM_OK;
     auto cleanup = [&]() {
@@ -1968,6 +1979,7 @@ int run_plan(asdm_cs &cs, const asdm_plan &plan, const asdm_run_opts &opt, asdm_
         dfree(d_ctr, s);
         dfree(d_local, s);
         dfree(d_rows, s);
+        dfree(d_field, s);
         dfree(d_mail, s);
     };
     EnumArgs a{};
@@ -1992,7 +2004,16 @@ int run_plan(asdm_cs &cs, const asdm_plan &plan, const asdm_run_opts &opt, asdm_
         }
         if (mode & ASDM_MODE_EMBED) {
             row_cap = opt.embeddings ? opt.emb_capacity : 0;
-            if ((rc = dalloc(&d_rows, std::max<uint64_t>(row_cap, 1) * n, s))) break;
+            lay = row_layout(cs);
+            std::vector<uint32_t> field(n);
+            for (uint32_t u = 0; u < n; ++u) field[u] = lay.word[u] << 8 | lay.shift[u];
+            if ((rc = dalloc(&d_rows, std::max<uint64_t>(row_cap, 1) * lay.words, s)) || (rc = dalloc(&d_field, n, s)))
+                break;
+            if (cudaMemcpyAsync(d_field, field.data(), n * sizeof(uint32_t), cudaMemcpyHostToDevice, s) != cudaSuccess ||
+                cudaStreamSynchronize(s) != cudaSuccess) {
+                rc = fail(ASDM_ERR_CUDA, "row layout upload failed");
+                break;
+            }
         }
         a.lv = reinterpret_cast<const DLevel *>(d_plan);
         a.bk = reinterpret_cast<const DBack *>(d_plan + n * sizeof(DLevel));
@@ -2006,6 +2027,8 @@ int run_plan(asdm_cs &cs, const asdm_plan &plan, const asdm_run_opts &opt, asdm_
         a.local = d_local;
         a.rows = d_rows;
         a.row_cap = row_cap;
+        a.field = d_field;
+        a.row_words = lay.words;
         a.mail = d_mail;
         a.limit_ns = opt.time_limit_s > 0 ? (uint64_t)(opt.time_limit_s * 1e9) : 0;
         a.count_limit = opt.count_limit;
@@ -2082,23 +2105,7 @@ int run_plan(asdm_cs &cs, const asdm_plan &plan, const asdm_run_opts &opt, asdm_
                           (unsigned long long)row_cap);
                 break;
             }
-            if (rows) {
-                std::vector<uint32_t> tmp(rows * n);
-                if (cudaMemcpyAsync(tmp.data(), d_rows, rows * n * sizeof(uint32_t), cudaMemcpyDeviceToHost, s) !=
-                        cudaSuccess ||
-                    cudaStreamSynchronize(s) != cudaSuccess) {
-                    rc = fail(ASDM_ERR_CUDA, "embedding readback failed");
-                    break;
-                }
-                std::vector<uint64_t> perm(rows);
-                std::iota(perm.begin(), perm.end(), 0ull);
-                std::sort(perm.begin(), perm.end(), [&](uint64_t x, uint64_t y) {
-                    return std::lexicographical_compare(tmp.begin() + x * n, tmp.begin() + x * n + n,
-                                                        tmp.begin() + y * n, tmp.begin() + y * n + n);
-                });
-                for (uint64_t r = 0; r < rows; ++r)
-                    std::memcpy(opt.embeddings + r * n, tmp.data() + perm[r] * n, n * sizeof(uint32_t));
-            }
+            if ((rc = sorted_rows(cs, lay, d_rows, row_cap, rows, opt.embeddings))) break;
         }
     } while (false);
     if (e0) cudaEventDestroy(e0);
