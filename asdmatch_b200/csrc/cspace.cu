@@ -451,9 +451,11 @@ __global__ void __launch_bounds__(kBlock) k3_write(const CompDesc *__restrict__ 
 // ---- K3b: candidate edges ---------------------------------------------------
 struct EdgeDesc {
     const uint32_t *cand_u;   // C(u)
-    const uint2 *cmem;        // per word of ranks in l(u2): {membership of C(u2), |C(u2)| before it}
+    uint32_t cmem;            // offset in the group's membership words: per word of ranks in l(u2),
+                              // {membership of C(u2), |C(u2)| before it}
     uint32_t ncand_u;
     uint32_t label_u2;
+    uint32_t pad;
 };
 
 // Index in C(u2) of the vertex of rank r in l(u2), or kNone (one 8-byte
@@ -468,6 +470,7 @@ __device__ __forceinline__ uint32_t cand_index(const uint2 *cm, uint32_t r) {
 // before cnt is overwritten with the count), both written by k3_bound.
 template <bool kFill>
 __global__ void __launch_bounds__(kBlock) k3_edges(DevGraph g, const EdgeDesc *__restrict__ edges,
+                                                   const uint2 *__restrict__ cmem,
                                                    const uint64_t *__restrict__ item_base, uint32_t nedges,
                                                    uint32_t *__restrict__ cnt, const uint64_t *__restrict__ wpos,
                                                    uint32_t *__restrict__ elist, unsigned long long *__restrict__ elems,
@@ -491,7 +494,7 @@ __global__ void __launch_bounds__(kBlock) k3_edges(DevGraph g, const EdgeDesc *_
                 const uint32_t i = (uint32_t)(item - item_base[ei]);
                 if (i < d.ncand_u) label_run(g, d.cand_u[i], d.label_u2, b, e);
             }
-            cm = d.cmem;
+            cm = cmem + d.cmem;
         }
         scanned += e - b;
         const bool coop = (e - b) > kLongRun;
@@ -533,100 +536,225 @@ __global__ void __launch_bounds__(kBlock) k3_edges(DevGraph g, const EdgeDesc *_
     }
 }
 
-// The padded fill with the neighbour scan spread over the lanes: a warp takes
-// 32 consecutive items and walks the concatenation of their label runs 32
-// entries at a time, a lane per entry, so every lane has a membership lookup
-// in flight whatever the run lengths.  In: cnt = run lengths, rstart = run
-// starts (k3_bound), upos = padded positions; out: each item's hits packed in
-// order at the front of its padded region, cnt = their number.
-__global__ void __launch_bounds__(kBlock, 6) k3_flat(DevGraph g, const EdgeDesc *__restrict__ edges,
-                                                  const uint64_t *__restrict__ item_base, uint32_t nedges,
-                                                  uint32_t *__restrict__ cnt, const uint64_t *__restrict__ upos,
-                                                  const uint32_t *__restrict__ rstart, uint32_t *__restrict__ padded,
-                                                  unsigned long long *__restrict__ elems) {
-    constexpr uint32_t kWarps = kBlock / 32;
-    __shared__ uint64_t s_pre[kWarps][33];   // exclusive prefix of the run lengths (s_pre[32] = total)
-    __shared__ uint64_t s_out[kWarps][32];   // padded position of each item
-    __shared__ const uint2 *s_cm[kWarps][32];
-    __shared__ uint32_t s_rs[kWarps][32], s_hits[kWarps][32];
-    const uint32_t lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    const uint64_t total = item_base[nedges];
-    const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
-    uint64_t scanned = 0;
-    for (uint64_t base = (uint64_t)blockIdx.x * blockDim.x + (threadIdx.x & ~31u); base < total; base += stride) {
-        const uint64_t item = base + lane;
-        uint64_t len = 0;
-        const uint32_t ei = warp_find_segment(item_base, nedges, base, item, item < total, lane);
-        if (item < total) {
-            s_cm[wid][lane] = edges[ei].cmem;
-            len = cnt[item];
-            s_rs[wid][lane] = rstart[item];
-            s_out[wid][lane] = upos[item];
-        }
-        uint64_t inc = len;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const uint64_t y = __shfl_up_sync(0xffffffffu, inc, o);
-            if (lane >= (uint32_t)o) inc += y;
-        }
-        s_pre[wid][lane + 1] = inc;
-        if (lane == 0) s_pre[wid][0] = 0;
-        s_hits[wid][lane] = 0;
-        __syncwarp();
-        const uint64_t S = s_pre[wid][32];
-        scanned += S;
-        // owner of entry j: the last item whose run starts at or before j
-        // (empty runs share their start with the next item and come first)
-        auto owner = [&](uint64_t j) {
-            uint32_t lo = 0, hi = 32;
-            while (hi - lo > 1) {
-                const uint32_t mid = (lo + hi) >> 1;
-                if (s_pre[wid][mid] <= j) lo = mid; else hi = mid;
-            }
-            return lo;
-        };
-        // one round's hits of the entries j0 .. j0+31 (idx = kNone for a miss)
-        // packed behind their item's earlier hits
-        auto emit = [&](uint64_t j0, uint32_t it, uint64_t first, uint32_t idx) {
-            const uint64_t j = j0 + lane;
-            const bool valid = j < S;
-            const uint32_t mask = __ballot_sync(0xffffffffu, idx != kNone);
-            // the item's lanes in this round are contiguous, from lane f
-            const uint32_t f = first > j0 ? (uint32_t)(first - j0) : 0u;
-            const uint32_t mine = mask & ~((1u << f) - 1u);
-            const uint32_t done = s_hits[wid][it];
-            if (idx != kNone) padded[s_out[wid][it] + done + __popc(mine & ((1u << lane) - 1u))] = idx;
-            const uint32_t next_it = __shfl_down_sync(0xffffffffu, it, 1);
-            const bool last = valid && (lane == 31 || j + 1 == S || next_it != it);
-            __syncwarp();
-            if (last) s_hits[wid][it] = done + __popc(mine & ((2u << lane) - 1u));
-            __syncwarp();
-        };
-        // two rounds at a time: both rounds' rank and membership loads are in
-        // flight together (the rounds' outputs are packed in order after)
-        for (uint64_t j0 = 0; j0 < S; j0 += 64) {
-            const uint64_t ja = j0 + lane, jb = ja + 32;
-            const bool va = ja < S, vb = jb < S;
-            const uint32_t ita = owner(ja), itb = owner(jb);
-            const uint64_t fa = s_pre[wid][ita], fb = s_pre[wid][itb];
-            const uint32_t ra = va ? g.nbr_rank[s_rs[wid][ita] + (uint32_t)(ja - fa)] : 0u;
-            const uint32_t rb = vb ? g.nbr_rank[s_rs[wid][itb] + (uint32_t)(jb - fb)] : 0u;
-            const uint32_t xa = va ? cand_index(s_cm[wid][ita], ra) : kNone;
-            const uint32_t xb = vb ? cand_index(s_cm[wid][itb], rb) : kNone;
-            emit(j0, ita, fa, xa);
-            if (j0 + 32 < S) emit(j0 + 32, itb, fb, xb);
-        }
-        if (item < total) cnt[item] = s_hits[wid][lane];
-        __syncwarp();
-    }
-    if (elems && lane == 0 && scanned) atomicAdd(elems, (unsigned long long)scanned);
+// The fill: every item's label run is scanned once.
+//
+// The entries of all runs, in item order, are cut into chunks of equal length, a
+// warp each, so hubs' runs spread over many warps.  A warp walks its chunk 32
+// entries at a time, a lane per entry, kRounds rounds' loads in flight
+// together; the items that start in a round are one bit mask (a warp
+// reduction), so an entry's owner is a population count.  Entries are in
+// output order, so the hits, packed by ballots, are the chunk's part of the
+// output as it stands: they go to the chunk's own place in a staging buffer,
+// and a prefix sum over the chunks' hits says where k3_pack copies them.
+//
+// Bound: the two dependent loads per entry (neighbour rank, membership word;
+// L2 hits mostly) and the instructions around them.  Measured on 512 queries
+// on 3.77M vertices (1.2 x 10^10 entries, 8.4 x 10^9 hits): a binary search
+// for every entry's owner in 64-bit positions 135 ms (and 36 ms for a packing
+// pass per item); tiles of a fixed number of items 275 ms (every block waits
+// for its hubs); chunks written at their final place after a look-back over
+// the chunks before them 84 ms with a look-back per block, 98 ms per warp
+// (thousands of chunks in flight to walk over).
+constexpr uint32_t kRounds = 4;
+// Entries per chunk, a power of two: finding its first items costs a chunk a
+// few dependent loads (512 queries as above: 83 ms with 512 entries, 69 ms
+// with 1,024, 61 ms with 2,048), but a small group needs its warps spread
+// (200 8-vertex queries on 3,112 vertices, 51,000 entries: 24 us with 512
+// entries, 63 us with 2,048), so chunks grow once every warp has two.
+constexpr uint32_t kChunkLog2Min = 7, kChunkLog2Max = 12;
+uint32_t chunk_log2_for(uint64_t entries, int num_sms) {
+    uint32_t k = kChunkLog2Min;
+    while (k < kChunkLog2Max && entries >> (k + 1) >= (uint64_t)num_sms * 64 * 2) ++k;
+    return k;
 }
 
-// Upper bound of every item's list: the length of the candidate's label run.
+struct FillWarp {
+    uint2 item[32];  // by rank among the batch's non-empty items: {entry number -> place in nbr_rank, cmem offset}
+};
+
+// The hits of 32 items (lane's item: entries nbr_rank[rs, rs + len),
+// membership words at cmem + cm), packed behind out; off = hits before this
+// lane's item.  Returns their number.
+__device__ __forceinline__ uint32_t fill_batch(const uint32_t *__restrict__ nbr_rank, const uint2 *__restrict__ cmem,
+                                               FillWarp &w, uint32_t lane, uint32_t rs, uint32_t len, uint32_t cm,
+                                               uint32_t *__restrict__ out, uint32_t &off) {
+    uint32_t inc = len;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t y = __shfl_up_sync(0xffffffffu, inc, o);
+        if (lane >= (uint32_t)o) inc += y;
+    }
+    const uint32_t start = inc - len, S = __shfl_sync(0xffffffffu, inc, 31);
+    const uint32_t lt = (1u << lane) - 1u, le = lt | (1u << lane);
+    const uint32_t some = __ballot_sync(0xffffffffu, len != 0);
+    if (len) w.item[__popc(some & lt)] = make_uint2(rs - start, cm);
+    __syncwarp();
+    uint32_t hits = 0, seen = 0;  // hits so far, non-empty items started so far
+    for (uint32_t j0 = 0; j0 < S; j0 += 32 * kRounds) {
+        uint2 it[kRounds], wd[kRounds];
+        uint32_t rank[kRounds];
+#pragma unroll
+        for (uint32_t r = 0; r < kRounds; ++r) {
+            const uint32_t d = start - (j0 + 32 * r);  // 32 or more when not in the round
+            const uint32_t heads = __reduce_or_sync(0xffffffffu, len && d < 32 ? 1u << d : 0u);
+            it[r] = w.item[seen + __popc(heads & le) - 1];
+            seen += __popc(heads);
+        }
+#pragma unroll
+        for (uint32_t r = 0; r < kRounds; ++r)  // lanes past the end repeat the last entry
+            rank[r] = nbr_rank[min(j0 + 32 * r + lane, S - 1) + it[r].x];
+#pragma unroll
+        for (uint32_t r = 0; r < kRounds; ++r) wd[r] = cmem[it[r].y + (rank[r] >> 5)];
+#pragma unroll
+        for (uint32_t r = 0; r < kRounds; ++r) {
+            const uint32_t bit = rank[r] & 31u;
+            const bool hit = ((wd[r].x >> bit) & 1u) && j0 + 32 * r + lane < S;
+            const uint32_t m = __ballot_sync(0xffffffffu, hit);
+            const uint32_t d = start - (j0 + 32 * r);
+            if (d < 32) off = hits + __popc(m & ((1u << d) - 1u));
+            if (hit) out[hits + __popc(m & lt)] = wd[r].y + __popc(wd[r].x & ((1u << bit) - 1u));
+            hits += __popc(m);
+        }
+    }
+    if (start >= S) off = hits;  // empty items after the last entry
+    __syncwarp();
+    return hits;
+}
+
+// The first item of every chunk (the one whose run holds the chunk's first
+// entry, or the first of the empty items at that place) and its edge.
+__global__ void __launch_bounds__(kBlock) k3_chunks(const uint64_t *__restrict__ item_base, uint32_t nedges,
+                                                    const uint64_t *__restrict__ upos, uint32_t chunk_log2,
+                                                    uint2 *__restrict__ chunk) {
+    const uint64_t total = item_base[nedges];
+    for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (uint64_t)gridDim.x * blockDim.x) {
+        const uint64_t s = upos[i], e = upos[i + 1];
+        uint64_t c = (s + (1ull << chunk_log2) - 1) >> chunk_log2;
+        if (c << chunk_log2 >= e) continue;
+        uint32_t f = (uint32_t)i, ei = find_segment(item_base, nedges, i);
+        for (; c << chunk_log2 < e; ++c) {
+            if (c << chunk_log2 == s) {
+                uint32_t b = f;
+                while (b > 0 && upos[b - 1] == s) --b;
+                chunk[c] = make_uint2(b, b == f ? ei : find_segment(item_base, nedges, b));
+            } else {
+                chunk[c] = make_uint2(f, ei);
+            }
+        }
+    }
+}
+
+// In: upos = prefix of the run lengths (nitems + 1), rstart = run starts, the
+// chunks' first items.  Out: the chunks' hits in stage, their numbers; eoff =
+// each item's position among its chunk's hits.
+__global__ void __launch_bounds__(kBlock, 5) k3_fill(DevGraph g, const EdgeDesc *__restrict__ edges,
+                                                  const uint2 *__restrict__ cmem,
+                                                  const uint64_t *__restrict__ item_base, uint32_t nedges,
+                                                  const uint64_t *__restrict__ upos, const uint32_t *__restrict__ rstart,
+                                                  const uint2 *__restrict__ chunk, uint32_t nchunks, uint32_t chunk_log2,
+                                                  uint32_t *__restrict__ eoff, uint32_t *__restrict__ stage,
+                                                  uint32_t *__restrict__ chunk_hits) {
+    __shared__ FillWarp s_warp[kBlock / 32];
+    const uint32_t lane = threadIdx.x & 31;
+    FillWarp &w = s_warp[threadIdx.x >> 5];
+    const uint32_t nitems = (uint32_t)item_base[nedges];
+    const uint64_t entries = upos[nitems];
+    const uint64_t nwarps = (uint64_t)gridDim.x * (kBlock / 32);
+    for (uint64_t c = (uint64_t)blockIdx.x * (kBlock / 32) + (threadIdx.x >> 5); c < nchunks; c += nwarps) {
+        const bool last = c + 1 == nchunks;
+        const uint64_t e0 = c << chunk_log2, e1 = last ? entries : e0 + (1ull << chunk_log2);
+        const uint2 p = chunk[c];
+        uint32_t base = p.x, edge = p.y, hits = 0;
+        uint64_t edge_end = item_base[edge + 1];
+        uint64_t s = base + lane < nitems ? upos[base + lane] : entries;
+        uint32_t rs = base + lane < nitems ? rstart[base + lane] : 0u;
+        for (;;) {
+            const uint32_t item = base + lane;
+            // the next 32 items, in flight while these are scanned
+            const bool more = (uint64_t)item + 32 < nitems;
+            const uint64_t s_next = more ? upos[item + 32] : entries;
+            const uint32_t rs_next = more ? rstart[item + 32] : 0u;
+            // this lane's edge: the warp's, or one of the next
+            uint32_t ei = edge;
+            if (item >= edge_end && item < nitems) ei = find_segment(item_base + edge, min(32u, nedges - edge), item) + edge;
+            const uint32_t cm = edges[ei].cmem;
+            const uint64_t after = __shfl_sync(0xffffffffu, s_next, 0);
+            uint64_t e = __shfl_down_sync(0xffffffffu, s, 1);
+            if (lane == 31) e = after;
+            const uint64_t lo = max(s, e0), hi = min(e, e1);
+            const uint32_t len = hi > lo ? (uint32_t)(hi - lo) : 0u;
+            uint32_t off = 0;
+            const uint32_t h = fill_batch(g.nbr_rank, cmem, w, lane, rs + (uint32_t)(lo - s), len, cm, stage + e0 + hits, off);
+            if (item < nitems && s >= e0 && (s < e1 || last)) eoff[item] = hits + off;
+            hits += h;
+            if ((uint64_t)base + 32 >= nitems || (after >= e1 && !last)) break;
+            base += 32;
+            s = s_next;
+            rs = rs_next;
+            edge = __shfl_sync(0xffffffffu, ei, 31);
+            edge_end = item_base[edge + 1];
+            if (edge_end <= base) edge_end = item_base[++edge + 1];  // lane 31 was its edge's last item
+        }
+        if (lane == 0) chunk_hits[c] = hits;
+    }
+}
+
+// The chunks' hits, side by side in elist: a warp per chunk, four entries a
+// lane in flight.
+__global__ void __launch_bounds__(kBlock) k3_pack(const uint32_t *__restrict__ stage, const uint32_t *__restrict__ chunk_hits,
+                                                  const uint64_t *__restrict__ chunk_base, uint32_t nchunks,
+                                                  uint32_t chunk_log2, uint32_t *__restrict__ elist) {
+    const uint32_t lane = threadIdx.x & 31;
+    const uint64_t nwarps = (uint64_t)gridDim.x * (kBlock / 32);
+    for (uint64_t c = (uint64_t)blockIdx.x * (kBlock / 32) + (threadIdx.x >> 5); c < nchunks; c += nwarps) {
+        const uint32_t n = chunk_hits[c];
+        const uint32_t *from = stage + (c << chunk_log2);
+        uint32_t *to = elist + chunk_base[c];
+        for (uint32_t i = lane; i < n; i += 128) {
+            uint32_t v[4];
+#pragma unroll
+            for (uint32_t k = 0; k < 4; ++k) v[k] = i + 32 * k < n ? from[i + 32 * k] : 0u;
+#pragma unroll
+            for (uint32_t k = 0; k < 4; ++k)
+                if (i + 32 * k < n) to[i + 32 * k] = v[k];
+        }
+    }
+}
+
+// Where an item's list starts in elist, from k3_fill's outputs.
+__device__ __forceinline__ unsigned long long list_start(const uint64_t *upos, uint32_t nchunks, uint32_t chunk_log2,
+                                                         const uint64_t *chunk_base, const uint32_t *eoff,
+                                                         uint64_t item) {
+    const uint64_t c = upos[item] >> chunk_log2;
+    return chunk_base[c < nchunks ? c : nchunks - 1] + eoff[item];
+}
+
+__global__ void k3_starts(const uint64_t *__restrict__ item_base, uint32_t nedges, const uint64_t *__restrict__ upos,
+                          uint32_t nchunks, uint32_t chunk_log2, const uint64_t *__restrict__ chunk_base,
+                          const uint32_t *__restrict__ eoff, uint64_t *__restrict__ edge_start) {
+    const uint32_t e = blockIdx.x * blockDim.x + threadIdx.x;
+    if (e < nedges) edge_start[e] = list_start(upos, nchunks, chunk_log2, chunk_base, eoff, item_base[e]);
+}
+
+// eoff relative to its edge's first entry (below 2^32: checked by the host)
+__global__ void __launch_bounds__(kBlock) k3_rebase(const uint64_t *__restrict__ item_base, uint32_t nedges,
+                                                    const uint64_t *__restrict__ upos, uint32_t nchunks, uint32_t chunk_log2,
+                                                    const uint64_t *__restrict__ chunk_base,
+                                                    const uint64_t *__restrict__ edge_start, uint32_t *__restrict__ eoff) {
+    const uint64_t total = item_base[nedges];
+    const uint32_t lane = threadIdx.x & 31;
+    for (uint64_t base = (uint64_t)blockIdx.x * blockDim.x + (threadIdx.x & ~31u); base < total;
+         base += (uint64_t)gridDim.x * blockDim.x) {
+        const uint64_t i = base + lane;
+        const uint32_t ei = warp_find_segment(item_base, nedges, base, i, i < total, lane);
+        if (i < total) eoff[i] = (uint32_t)(list_start(upos, nchunks, chunk_log2, chunk_base, eoff, i) - edge_start[ei]);
+    }
+}
+
+// Every item's label run: its length (the upper bound of its list) and start.
 __global__ void __launch_bounds__(kBlock) k3_bound(DevGraph g, const EdgeDesc *__restrict__ edges,
                                                    const uint64_t *__restrict__ item_base, uint32_t nedges,
-                                                   uint32_t *__restrict__ ub,
-                                                   uint32_t *__restrict__ rstart) {
+                                                   uint32_t *__restrict__ ub, uint32_t *__restrict__ rstart) {
     const uint64_t total = item_base[nedges];
     const uint32_t lane = threadIdx.x & 31;
     for (uint64_t base = (uint64_t)blockIdx.x * blockDim.x + (threadIdx.x & ~31u); base < total;
@@ -639,58 +767,7 @@ __global__ void __launch_bounds__(kBlock) k3_bound(DevGraph g, const EdgeDesc *_
         uint32_t b = 0, e = 0;
         if (i < d.ncand_u) label_run(g, d.cand_u[i], d.label_u2, b, e);
         ub[item] = e - b;
-        if (rstart) rstart[item] = b;
-    }
-}
-
-// Dense copy of the padded lists: a lane per item copies a short list, the
-// warp together copies every list longer than 32 entries.
-// The same pass turns the counts (cnt) into each item's offset within its
-// edge's list, records each edge's first entry and flags a list offset past
-// 2^32 (the work of k3_offsets).
-__global__ void __launch_bounds__(kBlock) k3_pack(const uint64_t *__restrict__ upos, uint32_t *__restrict__ cnt,
-                                                  const uint64_t *__restrict__ wpos, uint64_t nitems,
-                                                  const uint32_t *__restrict__ padded, uint32_t *__restrict__ elist,
-                                                  const uint64_t *__restrict__ item_base, uint32_t nedges,
-                                                  uint64_t *__restrict__ edge_start, uint32_t *__restrict__ bad) {
-    const uint32_t lane = threadIdx.x & 31;
-    const uint64_t nwarps = (uint64_t)gridDim.x * (blockDim.x >> 5);
-    for (uint64_t base = ((uint64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)) * 32; base < nitems;
-         base += nwarps * 32) {
-        const uint64_t my = base + lane;
-        const uint32_t c = my < nitems ? cnt[my] : 0u;
-        const uint64_t from = my < nitems ? upos[my] : 0, to = my < nitems ? wpos[my] : 0;
-        const uint32_t ei = warp_find_segment(item_base, nedges, base, my, my < nitems, lane);
-        if (my < nitems) {
-            const uint64_t first = item_base[ei];
-            const uint64_t rel = to - wpos[first];
-            if (rel > 0xFFFFFFFFull) atomicExch(bad, 1u);
-            cnt[my] = (uint32_t)rel;
-            if (my == first) edge_start[ei] = to;
-        }
-        // the 32 items' dense lists are one contiguous range from lane 0's
-        // position: the warp copies it a lane per entry (coalesced stores),
-        // each entry read from its owner item's padded list
-        uint64_t pre = c;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const uint64_t y = __shfl_up_sync(0xffffffffu, pre, o);
-            if (lane >= (uint32_t)o) pre += y;
-        }
-        const uint64_t total = __shfl_sync(0xffffffffu, pre, 31), to0 = __shfl_sync(0xffffffffu, to, 0);
-        for (uint64_t t0 = 0; t0 < total; t0 += 32) {
-            const uint64_t t = t0 + lane;
-            // owner: the first lane whose inclusive prefix passes t
-            uint32_t o = 0;
-#pragma unroll
-            for (uint32_t step = 16; step; step >>= 1) {
-                const uint64_t v = __shfl_sync(0xffffffffu, pre, o + step - 1);
-                if (v <= t) o += step;
-            }
-            const uint64_t f = __shfl_sync(0xffffffffu, from, o);
-            const uint64_t ex = __shfl_sync(0xffffffffu, pre - c, o);
-            if (t < total) elist[to0 + t] = padded[f + (t - ex)];
-        }
+        rstart[item] = b;
     }
 }
 
@@ -1183,7 +1260,8 @@ int build_batch(const std::vector<asdm_cs *> &group) {
             for (uint32_t e = q.off[u]; e < q.off[u + 1]; ++e) {
                 const uint32_t u2 = q.nbr[e];
                 const uint32_t s2 = qp.seg0 + u2;
-                edges.push_back(EdgeDesc{arena->d_cand + cs.cand_base[u], cmem + mword[s2], cs.ncand[u], q.lab[u2]});
+                edges.push_back(
+                    EdgeDesc{arena->d_cand + cs.cand_base[u], (uint32_t)mword[s2], cs.ncand[u], q.lab[u2], 0});
                 item_base.push_back(item_base.back() + cs.ncand[u] + 1);
             }
     }
@@ -1191,57 +1269,72 @@ int build_batch(const std::vector<asdm_cs *> &group) {
     const uint64_t nitems = item_base.back();
     std::vector<uint64_t> estart(ne, 0);
     bool two_scan = false;
-    uint64_t total = 0;
+    uint64_t total = 0, run_entries = 0;
     if (ne) {
         EdgeDesc *d_edges = nullptr;
         uint64_t *d_ib = nullptr, *d_wpos = nullptr, *d_estart = nullptr;
         uint32_t *d_bad = nullptr;
         ASDM_TRY(scr.upload(&d_edges, edges));
         ASDM_TRY(scr.upload(&d_ib, item_base));
-        ASDM_TRY(scr.alloc(&d_wpos, nitems + 1));
         ASDM_TRY(scr.alloc(&d_estart, ne));
         ASDM_TRY(scr.alloc(&d_bad, 1));
         ASDM_TRY(dalloc(&arena->d_eoff, nitems, s));
         ASDM_CUDA(cudaMemsetAsync(d_bad, 0, sizeof(uint32_t), s));
         const unsigned egrid = grid_for(nitems, G->num_sms);
-        // One scan of the neighbour runs: fill into lists padded to their
-        // label-run lengths (counting on the way), then pack densely; the
-        // exact two-scan form (count, then fill) where the padded lists would
-        // be too large.
+        // One scan of the neighbour runs into a staging buffer of their total
+        // length, packed densely after; the exact two-scan form (count, then fill) where that would
+        // be too large.  K3 keeps edge-major order: a warp's lanes take
+        // consecutive candidates of one edge, whose ascending ids put their
+        // adjacency runs side by side in the CSR (grouping by vertex block
+        // across edges measured slower).
         uint64_t bound = 0;
-        uint64_t *d_upos = nullptr;
-        // K3 keeps edge-major order: a warp's lanes take consecutive candidates
-        // of one edge, whose ascending ids put their adjacency runs side by
-        // side in the CSR (grouping by vertex block across edges measured slower)
-        ASDM_TRY(scr.alloc(&d_upos, nitems + 1));
         uint32_t *rstart = nullptr;
+        uint64_t *d_upos = nullptr;
         ASDM_TRY(scr.alloc(&rstart, nitems));
+        ASDM_TRY(scr.alloc(&d_upos, nitems + 1));
         k3_bound<<<egrid, kBlock, 0, s>>>(g, d_edges, d_ib, ne, arena->d_eoff, rstart);
         ::asdm::count_launch();
         ASDM_CUDA(cudaGetLastError());
         ASDM_TRY(scan_exclusive_u32(arena->d_eoff, d_upos, nitems, true, s));
         ASDM_CUDA(cudaMemcpyAsync(&bound, d_upos + nitems, sizeof(uint64_t), cudaMemcpyDeviceToHost, s));
         ASDM_CUDA(cudaStreamSynchronize(s));
-        // padded lists up to 2^padded_cap_log2 entries in total (default 2^33:
-        // 32 GiB), the exact two-scan form beyond
+        // staging buffers of up to 2^padded_cap_log2 entries (default 2^33: 32 GiB)
         const uint64_t padded_cap = 1ull << G->tuning.padded_cap_log2;
-        two_scan = bound > padded_cap;
-        if (bound <= padded_cap) {
-            uint32_t *padded = nullptr;
-            ASDM_TRY(scr.alloc(&padded, bound));
-            k3_flat<<<egrid, kBlock, 0, s>>>(g, d_edges, d_ib, ne, arena->d_eoff, d_upos, rstart, padded, d_elems + 1);
+        two_scan = bound > padded_cap || nitems >= 0xFFFFFF00ull;  // k3_fill numbers items in 32 bits
+        if (!two_scan) {
+            const uint32_t clog = chunk_log2_for(bound, G->num_sms);
+            const uint32_t nchunks = (uint32_t)std::max<uint64_t>(1, (bound + (1ull << clog) - 1) >> clog);
+            uint2 *d_chunk = nullptr;  // the chunks' first items
+            uint32_t *d_stage = nullptr, *d_chits = nullptr;
+            uint64_t *d_cbase = nullptr;
+            ASDM_TRY(scr.alloc(&d_stage, (uint64_t)nchunks << clog));
+            ASDM_TRY(scr.alloc(&d_chunk, nchunks));
+            ASDM_TRY(scr.alloc(&d_chits, nchunks));
+            ASDM_TRY(scr.alloc(&d_cbase, (uint64_t)nchunks + 1));
+            if (bound == 0) ASDM_CUDA(cudaMemsetAsync(d_chunk, 0, sizeof(uint2), s));
+            k3_chunks<<<egrid, kBlock, 0, s>>>(d_ib, ne, d_upos, clog, d_chunk);
+            ::asdm::count_launch();
+            const unsigned cgrid = grid_for(32ull * nchunks, G->num_sms);  // a warp per chunk
+            k3_fill<<<cgrid, kBlock, 0, s>>>(g, d_edges, cmem, d_ib, ne, d_upos, rstart, d_chunk, nchunks, clog,
+                                             arena->d_eoff, d_stage, d_chits);
             ::asdm::count_launch();
             ASDM_CUDA(cudaGetLastError());
-            ASDM_TRY(scan_exclusive_u32(arena->d_eoff, d_wpos, nitems, true, s));
-            ASDM_CUDA(cudaMemcpyAsync(&total, d_wpos + nitems, sizeof(uint64_t), cudaMemcpyDeviceToHost, s));
+            ASDM_TRY(scan_exclusive_u32(d_chits, d_cbase, nchunks, true, s));
+            ASDM_CUDA(cudaMemcpyAsync(&total, d_cbase + nchunks, sizeof(uint64_t), cudaMemcpyDeviceToHost, s));
+            k3_starts<<<(ne + kBlock - 1) / kBlock, kBlock, 0, s>>>(d_ib, ne, d_upos, nchunks, clog, d_cbase, arena->d_eoff,
+                                                                   d_estart);
+            ::asdm::count_launch();
+            k3_rebase<<<egrid, kBlock, 0, s>>>(d_ib, ne, d_upos, nchunks, clog, d_cbase, d_estart, arena->d_eoff);
+            ::asdm::count_launch();
             ASDM_CUDA(cudaStreamSynchronize(s));
             ASDM_TRY(dalloc(&arena->d_elist, total, s));
-            k3_pack<<<grid_for(nitems, G->num_sms), kBlock, 0, s>>>(d_upos, arena->d_eoff, d_wpos, nitems, padded,
-                                                                   arena->d_elist, d_ib, ne, d_estart, d_bad);
+            k3_pack<<<cgrid, kBlock, 0, s>>>(d_stage, d_chits, d_cbase, nchunks, clog, arena->d_elist);
             ::asdm::count_launch();
             ASDM_CUDA(cudaGetLastError());
+            run_entries = bound;
         } else {
-            k3_edges<false><<<egrid, kBlock, 0, s>>>(g, d_edges, d_ib, ne, arena->d_eoff, nullptr, nullptr,
+            ASDM_TRY(scr.alloc(&d_wpos, nitems + 1));
+            k3_edges<false><<<egrid, kBlock, 0, s>>>(g, d_edges, cmem, d_ib, ne, arena->d_eoff, nullptr, nullptr,
                                                     d_elems + 1, nullptr);
             ::asdm::count_launch();
             ASDM_CUDA(cudaGetLastError());
@@ -1249,7 +1342,7 @@ int build_batch(const std::vector<asdm_cs *> &group) {
             ASDM_CUDA(cudaMemcpyAsync(&total, d_wpos + nitems, sizeof(uint64_t), cudaMemcpyDeviceToHost, s));
             ASDM_CUDA(cudaStreamSynchronize(s));
             ASDM_TRY(dalloc(&arena->d_elist, total, s));
-            k3_edges<true><<<egrid, kBlock, 0, s>>>(g, d_edges, d_ib, ne, nullptr, d_wpos, arena->d_elist,
+            k3_edges<true><<<egrid, kBlock, 0, s>>>(g, d_edges, cmem, d_ib, ne, nullptr, d_wpos, arena->d_elist,
                                                     nullptr, nullptr);
             ::asdm::count_launch();
             ASDM_CUDA(cudaGetLastError());
@@ -1262,6 +1355,8 @@ int build_batch(const std::vector<asdm_cs *> &group) {
         ASDM_CUDA(cudaMemcpyAsync(estart.data(), d_estart, ne * sizeof(uint64_t), cudaMemcpyDeviceToHost, s));
         ASDM_CUDA(cudaMemcpyAsync(&bad, d_bad, sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
         ASDM_CUDA(cudaStreamSynchronize(s));
+        for (uint32_t e = 0; e < ne && !bad; ++e)
+            bad = (e + 1 < ne ? estart[e + 1] : total) - estart[e] > 0xFFFFFFFFull;
         if (bad) return fail(ASDM_ERR_INVALID, "a candidate-edge list exceeds 2^32 entries");
     }
     unsigned long long elems[2] = {0, 0};
@@ -1276,7 +1371,7 @@ int build_batch(const std::vector<asdm_cs *> &group) {
     // signature (and copies F words for the repeats); K2 and K3 read one rank
     // per scanned neighbour; compaction reads the bitsets it ANDs; K3 writes
     // the candidate-edge lists and their offsets (4 bytes per entry)
-    const uint64_t bytes = 8ull * seg.back() + 8ull * copied_words + 4ull * (elems[0] + elems[1]) +
+    const uint64_t bytes = 8ull * seg.back() + 8ull * copied_words + 4ull * (elems[0] + elems[1] + run_entries) +
                            4ull * bit_words_read + 4ull * total + 4ull * nitems;
     for (uint32_t qi = 0; qi < Q; ++qi) {
         QPlan &qp = P[qi];
