@@ -89,22 +89,31 @@ struct FilterArgs {
     const uint32_t *qnlc;     // (label, count) pairs
     const uint32_t *qnlc_off; // nseg + 1
     uint32_t nq;              // number of segments
+    uint32_t run_words;       // words per run
     uint32_t *fcount;         // |F(u)|
 };
 
-// A warp takes a run of up to kK1Words words (32 items each) inside one
+// A warp takes a run of up to run_words words (32 items each) inside one
 // segment, so the segment lookup and the query vertex's parameters are read
-// once per run.
-constexpr uint32_t kK1Words = 32;
+// once per run: 32 words where there are enough for every warp, fewer in
+// small groups (a run's words follow one another, about 1 us each: one
+// 8-vertex query on 3,112 vertices took 34 us with 32).
+constexpr uint32_t kMaxRunWords = 32;
+// Words per warp: a power of two up to kMaxRunWords that leaves every resident warp a run.
+uint32_t run_words_for(uint64_t words, int num_sms) {
+    uint32_t w = kMaxRunWords;
+    while (w > 1 && words < (uint64_t)num_sms * 64 * w) w >>= 1;
+    return w;
+}
 
 __global__ void __launch_bounds__(kBlock) k1_filter(FilterArgs a) {
     const uint64_t total_words = a.seg[a.nq] / 32;
     const uint32_t lane = threadIdx.x & 31;
     const uint64_t nwarps = (uint64_t)gridDim.x * (blockDim.x >> 5);
-    const uint64_t nruns = (total_words + kK1Words - 1) / kK1Words;
+    const uint64_t nruns = (total_words + a.run_words - 1) / a.run_words;
     for (uint64_t run = (uint64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); run < nruns; run += nwarps) {
-        uint64_t w = run * kK1Words;
-        const uint64_t w_end = min(total_words, w + kK1Words);
+        uint64_t w = run * a.run_words;
+        const uint64_t w_end = min(total_words, w + a.run_words);
         while (w < w_end) {
             const uint32_t u = find_segment(a.seg, a.nq, w * 32);
             const uint64_t seg_w0 = a.seg[u] / 32, seg_w1 = a.seg[u + 1] / 32;
@@ -156,87 +165,26 @@ __global__ void __launch_bounds__(kBlock) copy_words(const CopySeg *__restrict__
 }
 
 // ---- K2: neighbour marking passes -------------------------------------------
-// Push form (used for the phantom vertex 0 of a storage): every l(u)-neighbour
-// of a listed vertex gets its bit in u's slot bitset.
-struct PassDesc {
-    const uint32_t *src;   // vertex ids
-    uint32_t *mbits;       // u's bitset for p
-    uint32_t label;        // l(u)
-    uint32_t pad;
-    const uint32_t *cond;  // or null: the pass runs only where *cond is nonzero
-};
-
-__device__ __forceinline__ void mark(const DevGraph &g, uint32_t *mb, uint32_t k) {
-    const uint32_t r = g.nbr_rank[k];
-    atomicOr(&mb[r >> 5], 1u << (r & 31u));  // result unused: a fire-and-forget reduction
-}
-
-// A warp takes 32 items and marks the concatenation of their label runs 32
-// entries at a time, a lane per entry (every lane has a reduction to issue,
-// whatever the run lengths).
-__global__ void __launch_bounds__(kBlock) k2_pass(DevGraph g, const PassDesc *__restrict__ passes,
-                                                  const uint64_t *__restrict__ prefix, uint32_t npass,
-                                                  unsigned long long *__restrict__ elems) {
-    constexpr uint32_t kWarps = kBlock / 32;
-    __shared__ uint64_t s_pre[kWarps][33];   // exclusive prefix of the run lengths (s_pre[32] = total)
-    __shared__ uint32_t *s_mb[kWarps][32];
-    __shared__ uint32_t s_b[kWarps][32];
-    const uint64_t total = prefix[npass];
-    const uint32_t lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
-    uint64_t scanned = 0;
-    for (uint64_t base = (uint64_t)blockIdx.x * blockDim.x + (threadIdx.x & ~31u); base < total; base += stride) {
-        const uint64_t pos = base + lane;
-        uint32_t b = 0, e = 0;
-        if (pos < total) {
-            const uint64_t item = pos;
-            const uint32_t p = find_segment(prefix, npass, item);
-            const PassDesc d = passes[p];
-            if (!d.cond || *d.cond) label_run(g, d.src[item - prefix[p]], d.label, b, e);
-            s_mb[wid][lane] = d.mbits;
-        }
-        s_b[wid][lane] = b;
-        uint64_t inc = e - b;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const uint64_t y = __shfl_up_sync(0xffffffffu, inc, o);
-            if (lane >= (uint32_t)o) inc += y;
-        }
-        s_pre[wid][lane + 1] = inc;
-        if (lane == 0) s_pre[wid][0] = 0;
-        __syncwarp();
-        const uint64_t S = s_pre[wid][32];
-        scanned += S;
-        for (uint64_t j = lane; j < S; j += 32) {
-            // owner: the last item whose run starts at or before j
-            uint32_t lo = 0, hi = 32;
-            while (hi - lo > 1) {
-                const uint32_t mid = (lo + hi) >> 1;
-                if (s_pre[wid][mid] <= j) lo = mid; else hi = mid;
-            }
-            mark(g, s_mb[wid][lo], s_b[wid][lo] + (uint32_t)(j - s_pre[wid][lo]));
-        }
-        __syncwarp();
-    }
-    if (lane == 0 && scanned) atomicAdd(elems, (unsigned long long)scanned);
-}
-
 // Pull form of a marking pass (p -> u): the bit of each candidate x of u
 // (F(u) for passes from earlier BFS neighbours, Ctd(u) for the later ones:
 // the final AND discards the rest) is set when some neighbour of x with label
 // l(p) lies in Ctd(p).  Same bits on those candidates as pushing from S(p);
-// the phantom vertex 0 of S(p) is pushed separately.  A warp takes 32 words
-// of candidates; each lane scans one candidate's label run, stopping at its
-// first member of Ctd(p), and runs left open after kPullLane entries are
-// finished by the whole warp 32 entries at a time.
+// the phantom vertex 0 of S(p), where there is one (*ph, set when Ctd(p) was
+// formed: the waves run without host reads), is pushed by one more group of
+// the pass, which marks its neighbours of u's label.  A warp takes a group of
+// run_words words of candidates (run_words_for); each lane scans one
+// candidate's label run, stopping at its first member of Ctd(p), and runs left
+// open after kPullLane entries are finished by the whole warp 32 entries at a
+// time.
 struct PullDesc {
+    const uint32_t *ph;      // whether S(p) has the phantom vertex
     const uint32_t *xbits;   // candidates to test, by rank in l(u)
     uint32_t *mbits;         // u's slot bitset for p
     const uint32_t *sbits;   // membership of Ctd(p), by rank in l(p)
     uint32_t lbase;          // vbl_off[l(u)]
     uint32_t label;          // l(p)
     uint32_t words;          // words of xbits
-    uint32_t pad;
+    uint32_t label_u;        // l(u)
 };
 
 constexpr uint32_t kPullLane = 16;
@@ -263,7 +211,7 @@ __device__ __forceinline__ bool pull_member(const DevGraph &g, const uint32_t *s
 
 __global__ void __launch_bounds__(kBlock) k2_pull(DevGraph g, const PullDesc *__restrict__ passes,
                                                   const uint64_t *__restrict__ group_pre, uint32_t npass,
-                                                  unsigned long long *__restrict__ elems) {
+                                                  uint32_t run_words, unsigned long long *__restrict__ elems) {
     constexpr uint32_t kWarps = kBlock / 32;
     __shared__ uint32_t s_out[kWarps][32];
     const uint32_t lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
@@ -275,8 +223,21 @@ __global__ void __launch_bounds__(kBlock) k2_pull(DevGraph g, const PullDesc *__
     for (uint64_t grp = (uint64_t)blockIdx.x * kWarps + wid; grp < ngroups; grp += nwarps) {
         const uint32_t pi = find_segment(group_pre, npass, grp);
         const PullDesc d = passes[pi];
-        const uint32_t w0 = (uint32_t)(grp - group_pre[pi]) * 32;
-        const uint32_t f = (w0 + lane < d.words) ? d.xbits[w0 + lane] : 0u;
+        const uint32_t w0 = (uint32_t)(grp - group_pre[pi]) * run_words;
+        if (grp + 1 == group_pre[pi + 1]) {
+            // the pass's last group: the phantom vertex
+            if (*d.ph) {
+                uint32_t b, e;
+                label_run(g, 0, d.label_u, b, e);
+                for (uint32_t k = b + lane; k < e; k += 32) {
+                    const uint32_t r = g.nbr_rank[k];
+                    atomicOr(&d.mbits[r >> 5], 1u << (r & 31u));  // result unused: a fire-and-forget reduction
+                }
+                if (lane == 0) scanned += e - b;
+            }
+            continue;
+        }
+        const uint32_t f = (lane < run_words && w0 + lane < d.words) ? d.xbits[w0 + lane] : 0u;
         // inclusive prefix of the candidates per word
         uint32_t pre = __popc(f);
 #pragma unroll
@@ -351,17 +312,36 @@ struct CompDesc {
     uint32_t need;          // slots whose bitsets are required
     uint32_t len;           // |V_l(u)|
     uint32_t lbase;         // vbl_off[l(u)]
-    uint32_t phantom;       // append data vertex 0 when fewer than len survive
-    uint32_t pad;
-    uint2 *cmem;            // or null: per word of the result, {membership bits, result size before it}
-    uint32_t *sbits;        // or null: the result's membership bits alone
-    uint32_t *ph;           // or null: set to 1 when the phantom vertex was appended, else 0
+    uint2 *cmem;            // C(u): per word of the result, {membership bits, result size before it}
+    uint32_t *sbits;        // Ctd(u): the result's membership bits
+    uint32_t *ph;           // Ctd(u): set when fewer than len survive (the reference's zero-filled storage tail
+                            // then holds data vertex 0, the phantom)
 };
 
 __device__ __forceinline__ uint32_t comp_word(const CompDesc &d, uint32_t w) {
     uint32_t x = d.bits[w];
     for (uint32_t m = d.need; m && x; m &= m - 1) x &= d.bits[(uint64_t)__ffs(m) * d.words + w];
     return x;
+}
+
+// Ctd(u) of a wave: its membership words and phantom flag.  first: prefix of
+// the segments' words.
+__global__ void __launch_bounds__(kBlock) k2_and(const CompDesc *__restrict__ segs, const uint64_t *__restrict__ first,
+                                                 uint32_t nseg) {
+    const uint64_t total = first[nseg];
+    const uint32_t lane = threadIdx.x & 31;
+    for (uint64_t base = (uint64_t)blockIdx.x * blockDim.x + (threadIdx.x & ~31u); base < total;
+         base += (uint64_t)gridDim.x * blockDim.x) {
+        const uint64_t t = base + lane;
+        const uint32_t si = warp_find_segment(first, nseg, base, t, t < total, lane);
+        if (t >= total) continue;
+        const CompDesc d = segs[si];
+        const uint32_t w = (uint32_t)(t - first[si]);
+        const uint32_t x = comp_word(d, w);
+        d.sbits[w] = x;
+        const uint32_t left = d.len - 32 * w;  // items of this word and after it
+        if (x != (left >= 32 ? 0xFFFFFFFFu : (1u << left) - 1u) && *(volatile uint32_t *)d.ph == 0) *d.ph = 1;
+    }
 }
 
 __global__ void __launch_bounds__(kBlock) k3_count(const CompDesc *__restrict__ segs, const uint64_t *__restrict__ tile_first,
@@ -386,8 +366,7 @@ __global__ void __launch_bounds__(kBlock) k3_count(const CompDesc *__restrict__ 
     }
 }
 
-// Segment sidx writes to out + tile_pos[tile_first[sidx]] + sidx (one spare
-// slot per segment for the phantom vertex).
+// Segment sidx writes to out + tile_pos[tile_first[sidx]].
 __global__ void __launch_bounds__(kBlock) k3_write(const CompDesc *__restrict__ segs, const uint64_t *__restrict__ tile_first,
                                                    uint32_t nseg, const uint64_t *__restrict__ tile_pos,
                                                    const uint32_t *__restrict__ vbl, uint32_t *__restrict__ out,
@@ -424,28 +403,17 @@ __global__ void __launch_bounds__(kBlock) k3_write(const CompDesc *__restrict__ 
     }
     __syncthreads();
     const uint64_t seg_first = tile_pos[tile_first[sidx]];
-    uint32_t *o = out ? out + seg_first + sidx : nullptr;  // null: sizes and bitsets only
+    uint32_t *o = out + seg_first;
     uint32_t pos = (uint32_t)(tile_pos[t] - seg_first) + (warp ? wsum[warp - 1] : 0) + v - c;
 #pragma unroll
     for (int k = 0; k < kItems; ++k) {
         const uint32_t w = my + k;
         if (w >= d.words) break;
-        if (d.cmem) d.cmem[w] = make_uint2(x[k], pos);
-        if (d.sbits) d.sbits[w] = x[k];
-        if (o)
-            for (uint32_t y = x[k]; y; y &= y - 1) o[pos++] = vbl[d.lbase + 32 * w + (uint32_t)(__ffs(y) - 1)];
+        d.cmem[w] = make_uint2(x[k], pos);
+        for (uint32_t y = x[k]; y; y &= y - 1) o[pos++] = vbl[d.lbase + 32 * w + (uint32_t)(__ffs(y) - 1)];
     }
     // the last tile of a segment records the segment size
-    if (threadIdx.x == 0 && t + 1 == tile_first[sidx + 1]) {
-        uint32_t size = (uint32_t)(tile_pos[t + 1] - seg_first);
-        const bool ph = d.phantom && size < d.len;  // the reference's zero-filled storage tail
-        if (ph) {
-            if (o) o[size] = 0;
-            ++size;
-        }
-        if (d.ph) *d.ph = ph ? 1u : 0u;
-        seg_count[sidx] = size;
-    }
+    if (threadIdx.x == 0 && t + 1 == tile_first[sidx + 1]) seg_count[sidx] = (uint32_t)(tile_pos[t + 1] - seg_first);
 }
 
 // ---- K3b: candidate edges ---------------------------------------------------
@@ -792,127 +760,9 @@ unsigned grid_for(uint64_t items, int num_sms) {
     return (unsigned)std::max<uint64_t>(1, std::min<uint64_t>(blocks, (uint64_t)num_sms * 32));
 }
 
-// One compaction over the given segments into one new device buffer (*out,
-// the caller frees it): segment i's vertices at *out + start[i], size[i] of
-// them (plus, where asked, the phantom vertex).  With out null only the
-// segments' device outputs (bitsets, phantom flags) are produced, with no
-// wait for the device.
-int compact(asdm_graph *G, const std::vector<CompDesc> &segs, uint32_t **out, std::vector<uint64_t> &start,
-            std::vector<uint32_t> &sizes) {
-    cudaStream_t s = G->stream;
-    const uint32_t nseg = (uint32_t)segs.size();
-    if (out) *out = nullptr;
-    sizes.assign(nseg, 0);
-    start.assign(nseg, 0);
-    if (nseg == 0) return ASDM_OK;
-    std::vector<uint64_t> tile_first(nseg + 1, 0);
-    for (uint32_t i = 0; i < nseg; ++i) tile_first[i + 1] = tile_first[i] + (segs[i].words + kTile - 1) / kTile;
-    const uint64_t ntiles = tile_first[nseg];
-    CompDesc *d_segs = nullptr;
-    uint64_t *d_tf = nullptr, *d_pos = nullptr;
-    uint32_t *d_cnt = nullptr, *d_sc = nullptr;
-    int rc = ASDM_OK;
-    std::vector<uint64_t> pos(ntiles + 1, 0);
-    do {
-        if (ntiles == 0) {
-            if (out && (rc = dalloc(out, nseg, s))) break;
-            for (uint32_t i = 0; i < nseg; ++i) start[i] = i;
-            break;
-        }
-        if ((rc = dalloc(&d_segs, nseg, s)) || (rc = dalloc(&d_tf, nseg + 1, s)) || (rc = dalloc(&d_cnt, ntiles, s)) ||
-            (rc = dalloc(&d_pos, ntiles + 1, s)) || (rc = dalloc(&d_sc, nseg, s)))
-            break;
-        if (upload_async(G, d_segs, segs.data(), nseg * sizeof(CompDesc)) != cudaSuccess ||
-            upload_async(G, d_tf, tile_first.data(), (nseg + 1) * sizeof(uint64_t)) !=
-                cudaSuccess ||
-            cudaMemsetAsync(d_sc, 0, nseg * sizeof(uint32_t), s) != cudaSuccess) {
-            rc = fail(ASDM_ERR_CUDA, "compaction upload failed");
-            break;
-        }
-        k3_count<<<(unsigned)ntiles, kBlock, 0, s>>>(d_segs, d_tf, nseg, d_cnt);
-        ::asdm::count_launch();
-        if (cudaGetLastError() != cudaSuccess) { rc = fail(ASDM_ERR_CUDA, "compaction count failed"); break; }
-        if ((rc = scan_exclusive_u32(d_cnt, d_pos, ntiles, true, s))) break;
-        if (!out) {
-            // bitsets and flags only: nothing for the host to read back
-            k3_write<<<(unsigned)ntiles, kBlock, 0, s>>>(d_segs, d_tf, nseg, d_pos, G->d.vbl, nullptr, d_sc);
-            ::asdm::count_launch();
-            if (cudaGetLastError() != cudaSuccess) rc = fail(ASDM_ERR_CUDA, "compaction write failed");
-            break;
-        }
-        if (cudaMemcpyAsync(pos.data(), d_pos, (ntiles + 1) * sizeof(uint64_t), cudaMemcpyDeviceToHost, s) !=
-                cudaSuccess ||
-            cudaStreamSynchronize(s) != cudaSuccess) {
-            rc = fail(ASDM_ERR_CUDA, "compaction readback failed");
-            break;
-        }
-        if ((rc = dalloc(out, pos[ntiles] + nseg, s))) break;
-        k3_write<<<(unsigned)ntiles, kBlock, 0, s>>>(d_segs, d_tf, nseg, d_pos, G->d.vbl, *out, d_sc);
-        ::asdm::count_launch();
-        if (cudaGetLastError() != cudaSuccess) { rc = fail(ASDM_ERR_CUDA, "compaction write failed"); break; }
-        if (cudaMemcpyAsync(sizes.data(), d_sc, nseg * sizeof(uint32_t), cudaMemcpyDeviceToHost, s) != cudaSuccess ||
-            cudaStreamSynchronize(s) != cudaSuccess) {
-            rc = fail(ASDM_ERR_CUDA, "compaction size readback failed");
-            break;
-        }
-        for (uint32_t i = 0; i < nseg; ++i) start[i] = pos[tile_first[i]] + i;
-    } while (false);
-    dfree(d_segs, s); dfree(d_tf, s); dfree(d_cnt, s); dfree(d_pos, s); dfree(d_sc, s);
-    if (rc != ASDM_OK && out) dfree(*out, s);
-    return rc;
-}
-
-int run_passes(asdm_graph *G, const std::vector<PassDesc> &passes, const std::vector<uint64_t> &lens,
-               unsigned long long *d_elems) {
-    cudaStream_t s = G->stream;
-    const uint32_t np = (uint32_t)passes.size();
-    if (np == 0) return ASDM_OK;
-    std::vector<uint64_t> prefix(np + 1, 0);
-    for (uint32_t i = 0; i < np; ++i) prefix[i + 1] = prefix[i] + lens[i];
-    if (prefix[np] == 0) return ASDM_OK;
-    PassDesc *d_p = nullptr;
-    uint64_t *d_prefix = nullptr;
-    ASDM_TRY(dalloc(&d_p, np, s));
-    ASDM_TRY(dalloc(&d_prefix, np + 1, s));
-    ASDM_CUDA(upload_async(G, d_p, passes.data(), np * sizeof(PassDesc)));
-    ASDM_CUDA(upload_async(G, d_prefix, prefix.data(), (np + 1) * sizeof(uint64_t)));
-    int rc = ASDM_OK;
-    k2_pass<<<grid_for(prefix[np], G->num_sms), kBlock, 0, s>>>(G->d, d_p, d_prefix, np, d_elems);
-    ::asdm::count_launch();
-    if (cudaGetLastError() != cudaSuccess) rc = fail(ASDM_ERR_CUDA, "marking pass failed");
-    dfree(d_p, s);
-    dfree(d_prefix, s);
-    return rc;
-}
-
-// All pull passes of one phase in one launch.
-int run_pulls(asdm_graph *G, const std::vector<PullDesc> &pulls, unsigned long long *d_elems) {
-    cudaStream_t s = G->stream;
-    const uint32_t np = (uint32_t)pulls.size();
-    if (np == 0) return ASDM_OK;
-    std::vector<uint64_t> gpre(np + 1, 0);
-    for (uint32_t i = 0; i < np; ++i) gpre[i + 1] = gpre[i] + (pulls[i].words + 31) / 32;
-    if (gpre[np] == 0) return ASDM_OK;
-    PullDesc *d_p = nullptr;
-    uint64_t *d_pre = nullptr;
-    int rc = ASDM_OK;
-    do {
-        if ((rc = dalloc(&d_p, np, s)) || (rc = dalloc(&d_pre, np + 1, s))) break;
-        if (upload_async(G, d_p, pulls.data(), np * sizeof(PullDesc)) != cudaSuccess ||
-            upload_async(G, d_pre, gpre.data(), (np + 1) * sizeof(uint64_t)) != cudaSuccess) {
-            rc = fail(ASDM_ERR_CUDA, "pull-pass upload failed");
-            break;
-        }
-        const uint64_t blocks = (gpre[np] + kBlock / 32 - 1) / (kBlock / 32);
-        const unsigned grid = (unsigned)std::max<uint64_t>(1, std::min<uint64_t>(blocks, (uint64_t)G->num_sms * 32));
-        k2_pull<<<grid, kBlock, 0, s>>>(G->d, d_p, d_pre, np, d_elems);
-        ::asdm::count_launch();
-        if (cudaGetLastError() != cudaSuccess) rc = fail(ASDM_ERR_CUDA, "pull pass failed");
-    } while (false);
-    dfree(d_p, s);
-    dfree(d_pre, s);
-    return rc;
-}
+// Candidate arrays of at most this many entries in total are allocated for
+// their bound, |V_l(u)| each, so the host need not read their sizes first.
+constexpr uint64_t kCandBound = 1u << 20;
 
 struct Scratch {
     cudaStream_t s;
@@ -927,11 +777,33 @@ struct Scratch {
         if (rc == ASDM_OK) ptrs.push_back((void *)*p);
         return rc;
     }
+};
+
+// Descriptor arrays that go to the device in one allocation and one copy
+// (a copy costs the host about 5 us whatever its size).
+struct Blob {
+    std::vector<uint8_t> h;
+    uint8_t *d = nullptr;
     template <typename T>
-    int upload(T **p, const std::vector<T> &h) {
-        ASDM_TRY(alloc(p, h.size()));
-        if (!h.empty()) ASDM_CUDA(upload_async(G, *p, h.data(), h.size() * sizeof(T)));
+    size_t put(const std::vector<T> &v) {
+        const size_t at = (h.size() + 15) & ~size_t(15);
+        h.resize(at + v.size() * sizeof(T));
+        if (!v.empty()) std::memcpy(h.data() + at, v.data(), v.size() * sizeof(T));
+        return at;
+    }
+    size_t zeros(size_t bytes) {
+        const size_t at = (h.size() + 15) & ~size_t(15);
+        h.resize(at + bytes, 0);
+        return at;
+    }
+    int upload(Scratch &scr) {
+        ASDM_TRY(scr.alloc(&d, h.size()));
+        if (!h.empty()) ASDM_CUDA(upload_async(scr.G, d, h.data(), h.size()));
         return ASDM_OK;
+    }
+    template <typename T>
+    T *at(size_t o) const {
+        return reinterpret_cast<T *>(d + o);
     }
 };
 
@@ -1020,56 +892,43 @@ int build_batch(const std::vector<asdm_cs *> &group) {
     }
     const uint32_t nk1 = (uint32_t)lbase.size();
     kfword.push_back(0);
-    uint32_t *bits = nullptr, *d_fcount = nullptr, *d_lbase = nullptr, *d_llen = nullptr, *d_qdeg = nullptr,
-             *d_qnlc = nullptr, *d_qnlc_off = nullptr;
-    uint64_t *d_seg = nullptr, *d_fword = nullptr;
-    unsigned long long *d_elems = nullptr;
+    uint32_t *bits = nullptr;
     ASDM_TRY(scr.alloc(&bits, fword[nseg]));
     ASDM_CUDA(cudaMemsetAsync(bits, 0, std::max<uint64_t>(fword[nseg], 1) * sizeof(uint32_t), s));
-    if (lbase.empty()) {
-        lbase.push_back(0);
-        llen.push_back(0);
-        qdeg.push_back(0);
+    // F of the repeated signatures
+    std::vector<CopySeg> cps;
+    std::vector<uint64_t> cpre{0};
+    for (uint32_t sg = 0; sg < nseg; ++sg) {
+        const uint32_t k = k1_of[sg];
+        if (kfword[k] == fword[sg]) continue;  // the vertex K1 filtered
+        cps.push_back(CopySeg{bits + kfword[k], bits + fword[sg]});
+        cpre.push_back(cpre.back() + words[sg]);
     }
-    ASDM_TRY(scr.upload(&d_seg, seg));
-    ASDM_TRY(scr.upload(&d_fword, kfword));
-    ASDM_TRY(scr.upload(&d_lbase, lbase));
-    ASDM_TRY(scr.upload(&d_llen, llen));
-    ASDM_TRY(scr.upload(&d_qdeg, qdeg));
-    if (qnlc.empty()) qnlc.push_back(0);
-    ASDM_TRY(scr.upload(&d_qnlc, qnlc));
-    ASDM_TRY(scr.upload(&d_qnlc_off, qnlc_off));
-    ASDM_TRY(scr.alloc(&d_fcount, std::max<uint32_t>(nk1, 1)));
-    ASDM_TRY(scr.alloc(&d_elems, 2));
-    ASDM_CUDA(cudaMemsetAsync(d_fcount, 0, std::max<uint32_t>(nk1, 1) * sizeof(uint32_t), s));
-    ASDM_CUDA(cudaMemsetAsync(d_elems, 0, 2 * sizeof(unsigned long long), s));
+    const uint64_t copied_words = cpre.back();
+    Blob b1;
+    const size_t o_seg = b1.put(seg), o_fword = b1.put(kfword), o_lbase = b1.put(lbase), o_llen = b1.put(llen),
+                 o_qdeg = b1.put(qdeg), o_qnlc = b1.put(qnlc), o_qnlc_off = b1.put(qnlc_off), o_cps = b1.put(cps),
+                 o_cpre = b1.put(cpre), o_fcount = b1.zeros(std::max<uint32_t>(nk1, 1) * sizeof(uint32_t)),
+                 o_elems = b1.zeros(2 * sizeof(unsigned long long)),
+                 o_ph = b1.zeros(std::max<uint32_t>(nseg, 1) * sizeof(uint32_t)), o_bad = b1.zeros(sizeof(uint32_t));
+    ASDM_TRY(b1.upload(scr));
+    uint32_t *d_fcount = b1.at<uint32_t>(o_fcount), *d_ph = b1.at<uint32_t>(o_ph);
+    unsigned long long *d_elems = b1.at<unsigned long long>(o_elems);
     if (seg[nk1]) {
-        FilterArgs fa{g, bits, d_seg, d_fword, d_lbase, d_llen, d_qdeg, d_qnlc, d_qnlc_off, nk1, d_fcount};
-        k1_filter<<<grid_for(seg[nk1] / kK1Words, G->num_sms), kBlock, 0, s>>>(fa);
+        const uint64_t kwords = seg[nk1] / 32;
+        const uint32_t rw = run_words_for(kwords, G->num_sms);
+        FilterArgs fa{g, bits, b1.at<uint64_t>(o_seg), b1.at<uint64_t>(o_fword), b1.at<uint32_t>(o_lbase),
+                      b1.at<uint32_t>(o_llen), b1.at<uint32_t>(o_qdeg), b1.at<uint32_t>(o_qnlc),
+                      b1.at<uint32_t>(o_qnlc_off), nk1, rw, d_fcount};
+        k1_filter<<<grid_for((kwords + rw - 1) / rw * 32, G->num_sms), kBlock, 0, s>>>(fa);  // a warp per run
         ::asdm::count_launch();
         ASDM_CUDA(cudaGetLastError());
     }
-    uint64_t copied_words = 0;
-    {
-        // F of the repeated signatures
-        std::vector<CopySeg> cps;
-        std::vector<uint64_t> cpre{0};
-        for (uint32_t sg = 0; sg < nseg; ++sg) {
-            const uint32_t k = k1_of[sg];
-            if (kfword[k] == fword[sg]) continue;  // the vertex K1 filtered
-            cps.push_back(CopySeg{bits + kfword[k], bits + fword[sg]});
-            cpre.push_back(cpre.back() + words[sg]);
-        }
-        copied_words = cpre.back();
-        if (!cps.empty() && cpre.back()) {
-            CopySeg *d_cps = nullptr;
-            uint64_t *d_cpre = nullptr;
-            ASDM_TRY(scr.upload(&d_cps, cps));
-            ASDM_TRY(scr.upload(&d_cpre, cpre));
-            copy_words<<<grid_for(cpre.back(), G->num_sms), kBlock, 0, s>>>(d_cps, d_cpre, (uint32_t)cps.size());
-            ::asdm::count_launch();
-            ASDM_CUDA(cudaGetLastError());
-        }
+    if (copied_words) {
+        copy_words<<<grid_for(copied_words, G->num_sms), kBlock, 0, s>>>(b1.at<CopySeg>(o_cps), b1.at<uint64_t>(o_cpre),
+                                                                        (uint32_t)cps.size());
+        ::asdm::count_launch();
+        ASDM_CUDA(cudaGetLastError());
     }
     std::vector<uint32_t> kcount(std::max<uint32_t>(nk1, 1), 0), fcount(nseg, 0);
     ASDM_CUDA(cudaMemcpyAsync(kcount.data(), d_fcount, kcount.size() * sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
@@ -1137,31 +996,44 @@ int build_batch(const std::vector<asdm_cs *> &group) {
     // storage S(u) scanned by the reference gets the phantom vertex 0)
     std::vector<uint64_t> mword(nseg + 1, 0);
     for (uint32_t i = 0; i < nseg; ++i) mword[i + 1] = mword[i] + words[i];
-    uint32_t *sbits = nullptr, *d_zero = nullptr, *d_ph = nullptr;
+    // (d_ph).  The waves' descriptors, the later passes' and the final
+    // compaction's go up together: no host read lies between them.
+    uint32_t *sbits = nullptr;
+    uint2 *cmem = nullptr;
     ASDM_TRY(scr.alloc(&sbits, std::max<uint64_t>(mword[nseg], 1)));
-    ASDM_TRY(scr.alloc(&d_zero, 1));
-    ASDM_TRY(scr.alloc(&d_ph, std::max<uint32_t>(nseg, 1)));
-    ASDM_CUDA(cudaMemsetAsync(d_zero, 0, sizeof(uint32_t), s));
-    ASDM_CUDA(cudaMemsetAsync(d_ph, 0, std::max<uint32_t>(nseg, 1) * sizeof(uint32_t), s));
+    ASDM_TRY(scr.alloc(&cmem, mword[nseg]));
     uint64_t bit_words_read = 0;
-    // a pass p -> u: pulled over u's candidates, plus the push of the phantom
-    // vertex, which runs where S(p) has it (a flag the compaction of Ctd(p)
-    // sets on the device: the waves run without host reads)
-    auto add_pass = [&](std::vector<PullDesc> &pulls, std::vector<PassDesc> &pushes, std::vector<uint64_t> &lens,
-                        const QPlan &qp, uint32_t u, uint32_t e, const uint32_t *xbits) {
+    struct Wave {
+        uint32_t npull = 0, nand = 0, run_words = 1;
+        uint64_t groups = 0, words = 0;
+        size_t o_pull = 0, o_gpre = 0, o_and = 0, o_wpre = 0;
+    };
+    Blob b2;
+    std::vector<PullDesc> pulls;
+    // a pass p -> u, pulled over u's candidates (and the phantom's push)
+    auto add_pass = [&](const QPlan &qp, uint32_t u, uint32_t e, const uint32_t *xbits) {
         const QueryGraph &q = qp.cs->q;
         const uint32_t p = q.nbr[e], su = qp.seg0 + u, sp = qp.seg0 + p, slot = e - q.off[u];
         uint32_t *mb = bits + fword[su] + (1ull + slot) * words[su];
-        pulls.push_back(PullDesc{xbits, mb, sbits + mword[sp], qp.lbase[u], q.lab[p], words[su], 0});
+        pulls.push_back(PullDesc{d_ph + sp, xbits, mb, sbits + mword[sp], qp.lbase[u], q.lab[p], words[su], q.lab[u]});
         bit_words_read += words[su];
-        pushes.push_back(PassDesc{d_zero, mb, q.lab[u], 0, d_ph + sp});
-        lens.push_back(1);
     };
+    auto put_pulls = [&](Wave &wv) {
+        uint64_t all = 0;
+        for (const PullDesc &d : pulls) all += d.words;
+        wv.run_words = run_words_for(all, G->num_sms);
+        std::vector<uint64_t> gpre{0};
+        for (const PullDesc &d : pulls) gpre.push_back(gpre.back() + (d.words + wv.run_words - 1) / wv.run_words + 1);
+        wv.npull = (uint32_t)pulls.size();
+        wv.groups = gpre.back();
+        wv.o_pull = b2.put(pulls);
+        wv.o_gpre = b2.put(gpre);
+        pulls.clear();
+    };
+    std::vector<Wave> waves(maxwave + 2);
     for (uint32_t w = 0; w <= maxwave; ++w) {
-        std::vector<PullDesc> pulls;
-        std::vector<PassDesc> pushes;
-        std::vector<uint64_t> lens;
-        std::vector<CompDesc> segs;
+        std::vector<CompDesc> ands;
+        std::vector<uint64_t> wpre{0};
         for (const QPlan &qp : P) {
             if (qp.empty) continue;
             const QueryGraph &q = qp.cs->q;
@@ -1172,66 +1044,100 @@ int build_batch(const std::vector<asdm_cs *> &group) {
                 for (uint32_t e = q.off[u]; e < q.off[u + 1]; ++e) {
                     if (qp.rank[q.nbr[e]] >= qp.rank[u]) continue;
                     need |= 1u << (e - q.off[u]);
-                    add_pass(pulls, pushes, lens, qp, u, e, bits + fword[su]);  // over F(u)
+                    add_pass(qp, u, e, bits + fword[su]);  // over F(u)
                 }
-                segs.push_back(CompDesc{bits + fword[su], words[su], need, qp.lsize[u], qp.lbase[u], 1, 0, nullptr,
+                ands.push_back(CompDesc{bits + fword[su], words[su], need, qp.lsize[u], qp.lbase[u], nullptr,
                                         sbits + mword[su], d_ph + su});
+                wpre.push_back(wpre.back() + words[su]);
                 bit_words_read += (uint64_t)(1 + __builtin_popcount(need)) * words[su];
             }
         }
-        ASDM_TRY(run_pulls(G, pulls, d_elems));
-        ASDM_TRY(run_passes(G, pushes, lens, d_elems));
-        std::vector<uint64_t> start;
-        std::vector<uint32_t> sizes;
-        ASDM_TRY(compact(G, segs, nullptr, start, sizes));  // Ctd(u) bitsets and phantom flags only
+        put_pulls(waves[w]);
+        waves[w].nand = (uint32_t)ands.size();
+        waves[w].words = wpre.back();
+        waves[w].o_and = b2.put(ands);
+        waves[w].o_wpre = b2.put(wpre);
     }
     // remaining passes (neighbours later in the BFS order), all queries at
-    // once, over Ctd(u)
-    {
-        std::vector<PullDesc> pulls;
-        std::vector<PassDesc> pushes;
-        std::vector<uint64_t> lens;
-        for (const QPlan &qp : P) {
-            if (qp.empty) continue;
-            const QueryGraph &q = qp.cs->q;
-            for (uint32_t u = 0; u < q.n; ++u)
-                for (uint32_t e = q.off[u]; e < q.off[u + 1]; ++e) {
-                    if (qp.rank[q.nbr[e]] < qp.rank[u]) continue;
-                    add_pass(pulls, pushes, lens, qp, u, e, sbits + mword[qp.seg0 + u]);
-                }
+    // once, over Ctd(u); then the final candidate sets, with the membership
+    // words and per-word prefix counts that K3 looks indices up in
+    std::vector<CompDesc> segs;
+    std::vector<uint32_t> seg_ids;
+    std::vector<uint64_t> tile_first{0};
+    uint64_t cand_bound = 0;
+    for (const QPlan &qp : P) {
+        if (qp.empty) continue;
+        const QueryGraph &q = qp.cs->q;
+        for (uint32_t u = 0; u < q.n; ++u) {
+            const uint32_t su = qp.seg0 + u;
+            for (uint32_t e = q.off[u]; e < q.off[u + 1]; ++e)
+                if (qp.rank[q.nbr[e]] >= qp.rank[u]) add_pass(qp, u, e, sbits + mword[su]);
+            const uint32_t all = q.deg(u) ? ((q.deg(u) == 32 ? 0xFFFFFFFFu : (1u << q.deg(u)) - 1u)) : 0u;
+            segs.push_back(CompDesc{bits + fword[su], words[su], all, qp.lsize[u], qp.lbase[u], cmem + mword[su],
+                                    nullptr, nullptr});
+            seg_ids.push_back(su);
+            tile_first.push_back(tile_first.back() + (words[su] + kTile - 1) / kTile);
+            cand_bound += qp.lsize[u];
+            bit_words_read += (uint64_t)(1 + q.deg(u)) * words[su];
         }
-        ASDM_TRY(run_pulls(G, pulls, d_elems));
-        ASDM_TRY(run_passes(G, pushes, lens, d_elems));
     }
-    // final candidate sets into the group's arena, with the membership
-    // bitsets and per-word prefix counts that K3 looks indices up in
+    put_pulls(waves[maxwave + 1]);
+    const uint32_t nfinal = (uint32_t)segs.size();
+    const uint64_t ntiles = tile_first.back();
+    const size_t o_segs = b2.put(segs), o_tf = b2.put(tile_first);
+    ASDM_TRY(b2.upload(scr));
+    for (const Wave &wv : waves) {
+        if (wv.npull) {
+            k2_pull<<<grid_for(32 * wv.groups, G->num_sms), kBlock, 0, s>>>(g, b2.at<PullDesc>(wv.o_pull),
+                                                                            b2.at<uint64_t>(wv.o_gpre), wv.npull,
+                                                                            wv.run_words, d_elems);
+            ::asdm::count_launch();
+        }
+        if (wv.words) {
+            k2_and<<<grid_for(wv.words, G->num_sms), kBlock, 0, s>>>(b2.at<CompDesc>(wv.o_and), b2.at<uint64_t>(wv.o_wpre),
+                                                                     wv.nand);
+            ::asdm::count_launch();
+        }
+    }
+    ASDM_CUDA(cudaGetLastError());
     auto arena = std::make_shared<CsArena>();
     arena->stream = s;
-    uint2 *cmem = nullptr;
-    ASDM_TRY(scr.alloc(&cmem, mword[nseg]));
     {
-        std::vector<CompDesc> segs;
-        std::vector<uint32_t> seg_ids;
-        for (const QPlan &qp : P) {
-            if (qp.empty) continue;
-            const QueryGraph &q = qp.cs->q;
-            for (uint32_t u = 0; u < q.n; ++u) {
-                const uint32_t all = q.deg(u) ? ((q.deg(u) == 32 ? 0xFFFFFFFFu : (1u << q.deg(u)) - 1u)) : 0u;
-                const uint32_t su = qp.seg0 + u;
-                segs.push_back(CompDesc{bits + fword[su], words[su], all, qp.lsize[u], qp.lbase[u], 0, 0,
-                                        cmem + mword[su]});
-                seg_ids.push_back(su);
-                bit_words_read += (uint64_t)(1 + q.deg(u)) * words[su];
+        std::vector<uint64_t> pos(ntiles + 1, 0);
+        std::vector<uint32_t> sizes(nfinal, 0);
+        if (ntiles) {
+            uint32_t *d_cnt = nullptr, *d_sc = nullptr;
+            uint64_t *d_pos = nullptr;
+            ASDM_TRY(scr.alloc(&d_cnt, ntiles));
+            ASDM_TRY(scr.alloc(&d_pos, ntiles + 1 + (nfinal + 1) / 2));  // positions, then the segments' sizes
+            d_sc = reinterpret_cast<uint32_t *>(d_pos + ntiles + 1);
+            k3_count<<<(unsigned)ntiles, kBlock, 0, s>>>(b2.at<CompDesc>(o_segs), b2.at<uint64_t>(o_tf), nfinal, d_cnt);
+            ::asdm::count_launch();
+            ASDM_CUDA(cudaGetLastError());
+            ASDM_TRY(scan_exclusive_u32(d_cnt, d_pos, ntiles, true, s));
+            uint64_t room = cand_bound;
+            if (cand_bound > kCandBound) {
+                ASDM_CUDA(cudaMemcpyAsync(&room, d_pos + ntiles, sizeof(uint64_t), cudaMemcpyDeviceToHost, s));
+                ASDM_CUDA(cudaStreamSynchronize(s));
             }
+            ASDM_TRY(dalloc(&arena->d_cand, room, s));
+            k3_write<<<(unsigned)ntiles, kBlock, 0, s>>>(b2.at<CompDesc>(o_segs), b2.at<uint64_t>(o_tf), nfinal, d_pos,
+                                                        g.vbl, arena->d_cand, d_sc);
+            ::asdm::count_launch();
+            ASDM_CUDA(cudaGetLastError());
+            std::vector<uint64_t> back(ntiles + 1 + (nfinal + 1) / 2);
+            ASDM_CUDA(cudaMemcpyAsync(back.data(), d_pos, back.size() * sizeof(uint64_t), cudaMemcpyDeviceToHost, s));
+            ASDM_CUDA(cudaStreamSynchronize(s));
+            std::copy(back.begin(), back.begin() + ntiles + 1, pos.begin());
+            const uint32_t *sc = reinterpret_cast<const uint32_t *>(back.data() + ntiles + 1);
+            for (uint32_t i = 0; i < nfinal; ++i)
+                sizes[i] = tile_first[i + 1] > tile_first[i] ? sc[i] : 0;  // a label without vertices has no tile
         }
-        std::vector<uint64_t> start;
-        std::vector<uint32_t> sizes;
-        ASDM_TRY(compact(G, segs, &arena->d_cand, start, sizes));
         std::vector<uint32_t> ncand(nseg, 0);
         std::vector<uint64_t> cbase(nseg, 0);
         for (size_t i = 0; i < seg_ids.size(); ++i) {
             ncand[seg_ids[i]] = sizes[i];
-            cbase[seg_ids[i]] = start[i];
+            cbase[seg_ids[i]] = pos[tile_first[i]];
         }
         if (!arena->d_cand) ASDM_TRY(dalloc(&arena->d_cand, 1, s));
         for (QPlan &qp : P) {
@@ -1271,15 +1177,15 @@ int build_batch(const std::vector<asdm_cs *> &group) {
     bool two_scan = false;
     uint64_t total = 0, run_entries = 0;
     if (ne) {
-        EdgeDesc *d_edges = nullptr;
-        uint64_t *d_ib = nullptr, *d_wpos = nullptr, *d_estart = nullptr;
-        uint32_t *d_bad = nullptr;
-        ASDM_TRY(scr.upload(&d_edges, edges));
-        ASDM_TRY(scr.upload(&d_ib, item_base));
+        Blob b3;
+        const size_t o_edges = b3.put(edges), o_ib = b3.put(item_base);
+        ASDM_TRY(b3.upload(scr));
+        const EdgeDesc *d_edges = b3.at<EdgeDesc>(o_edges);
+        const uint64_t *d_ib = b3.at<uint64_t>(o_ib);
+        uint64_t *d_wpos = nullptr, *d_estart = nullptr;
+        uint32_t *d_bad = b1.at<uint32_t>(o_bad);
         ASDM_TRY(scr.alloc(&d_estart, ne));
-        ASDM_TRY(scr.alloc(&d_bad, 1));
         ASDM_TRY(dalloc(&arena->d_eoff, nitems, s));
-        ASDM_CUDA(cudaMemsetAsync(d_bad, 0, sizeof(uint32_t), s));
         const unsigned egrid = grid_for(nitems, G->num_sms);
         // One scan of the neighbour runs into a staging buffer of their total
         // length, packed densely after; the exact two-scan form (count, then fill) where that would
@@ -1353,7 +1259,7 @@ int build_batch(const std::vector<asdm_cs *> &group) {
         }
         uint32_t bad = 0;
         ASDM_CUDA(cudaMemcpyAsync(estart.data(), d_estart, ne * sizeof(uint64_t), cudaMemcpyDeviceToHost, s));
-        ASDM_CUDA(cudaMemcpyAsync(&bad, d_bad, sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
+        if (two_scan) ASDM_CUDA(cudaMemcpyAsync(&bad, d_bad, sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
         ASDM_CUDA(cudaStreamSynchronize(s));
         for (uint32_t e = 0; e < ne && !bad; ++e)
             bad = (e + 1 < ne ? estart[e + 1] : total) - estart[e] > 0xFFFFFFFFull;

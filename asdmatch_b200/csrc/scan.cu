@@ -13,7 +13,8 @@ constexpr int kTile = kThreads * kItems;
 
 template <typename Tin>
 __global__ void __launch_bounds__(kThreads) scan_tiles(const Tin *__restrict__ in, uint64_t *__restrict__ out,
-                                                     uint64_t *__restrict__ tile_sums, uint64_t n) {
+                                                     uint64_t *__restrict__ tile_sums, uint64_t *__restrict__ total,
+                                                     uint64_t n) {
     __shared__ uint64_t stage[kTile];
     __shared__ uint64_t warp_tot[kThreads / 32];
     const uint64_t base = (uint64_t)blockIdx.x * kTile;
@@ -58,10 +59,15 @@ __global__ void __launch_bounds__(kThreads) scan_tiles(const Tin *__restrict__ i
         uint64_t idx = base + i;
         if (idx < n) out[idx] = stage[i];
     }
-    if (threadIdx.x == kThreads - 1) tile_sums[blockIdx.x] = prefix + tsum;
+    if (threadIdx.x == kThreads - 1) {
+        if (tile_sums) tile_sums[blockIdx.x] = prefix + tsum;
+        if (total) *total = prefix + tsum;  // a single tile
+    }
 }
 
-__global__ void add_tile_prefix(uint64_t *__restrict__ out, const uint64_t *__restrict__ tile_prefix, uint64_t n) {
+__global__ void add_tile_prefix(uint64_t *__restrict__ out, const uint64_t *__restrict__ tile_prefix, uint64_t n,
+                                uint64_t *__restrict__ total) {
+    if (total && blockIdx.x == 0 && threadIdx.x == 0) *total = tile_prefix[gridDim.x];
     const uint64_t base = (uint64_t)blockIdx.x * kTile;
     const uint64_t add = tile_prefix[blockIdx.x];
     for (int i = threadIdx.x; i < kTile; i += blockDim.x) {
@@ -77,32 +83,25 @@ int scan_impl(const Tin *in, uint64_t *out, uint64_t n, bool with_total, cudaStr
         return ASDM_OK;
     }
     const uint64_t ntiles = (n + kTile - 1) / kTile;
-    uint64_t *sums = nullptr;
-    ASDM_TRY(dalloc(&sums, ntiles + 1, s));
-    scan_tiles<Tin><<<(unsigned)ntiles, kThreads, 0, s>>>(in, out, sums, n);
-    ::asdm::count_launch();
-    ASDM_CUDA(cudaGetLastError());
-    int rc = ASDM_OK;
-    uint64_t *prefix = nullptr;
+    uint64_t *total = with_total ? out + n : nullptr;
     if (ntiles == 1) {
-        // single tile: its sum is the total
-        if (with_total) {
-            cudaError_t e = cudaMemcpyAsync(out + n, sums, sizeof(uint64_t), cudaMemcpyDeviceToDevice, s);
-            if (e != cudaSuccess) rc = fail(ASDM_ERR_CUDA, "scan total copy: %s", cudaGetErrorString(e));
-        }
-    } else {
-        // exclusive scan of the tile sums, grand total in prefix[ntiles]
-        rc = dalloc(&prefix, ntiles + 1, s);
-        if (rc == ASDM_OK) rc = scan_impl<uint64_t>(sums, prefix, ntiles, true, s);
-        if (rc == ASDM_OK) {
-            add_tile_prefix<<<(unsigned)ntiles, kThreads, 0, s>>>(out, prefix, n);
-            ::asdm::count_launch();
-            if (cudaGetLastError() != cudaSuccess) rc = fail(ASDM_ERR_CUDA, "scan launch failed");
-        }
-        if (rc == ASDM_OK && with_total) {
-            cudaError_t e = cudaMemcpyAsync(out + n, prefix + ntiles, sizeof(uint64_t), cudaMemcpyDeviceToDevice, s);
-            if (e != cudaSuccess) rc = fail(ASDM_ERR_CUDA, "scan total copy: %s", cudaGetErrorString(e));
-        }
+        scan_tiles<Tin><<<1, kThreads, 0, s>>>(in, out, nullptr, total, n);
+        ::asdm::count_launch();
+        ASDM_CUDA(cudaGetLastError());
+        return ASDM_OK;
+    }
+    uint64_t *sums = nullptr, *prefix = nullptr;
+    ASDM_TRY(dalloc(&sums, ntiles, s));
+    scan_tiles<Tin><<<(unsigned)ntiles, kThreads, 0, s>>>(in, out, sums, nullptr, n);
+    ::asdm::count_launch();
+    int rc = cudaGetLastError() == cudaSuccess ? ASDM_OK : fail(ASDM_ERR_CUDA, "scan launch failed");
+    // exclusive scan of the tile sums, grand total in prefix[ntiles]
+    if (rc == ASDM_OK) rc = dalloc(&prefix, ntiles + 1, s);
+    if (rc == ASDM_OK) rc = scan_impl<uint64_t>(sums, prefix, ntiles, true, s);
+    if (rc == ASDM_OK) {
+        add_tile_prefix<<<(unsigned)ntiles, kThreads, 0, s>>>(out, prefix, n, total);
+        ::asdm::count_launch();
+        if (cudaGetLastError() != cudaSuccess) rc = fail(ASDM_ERR_CUDA, "scan launch failed");
     }
     dfree(prefix, s);
     dfree(sums, s);
