@@ -67,7 +67,7 @@ extern "C" int asdm_gemm_bf16(int M, int N, int K, const uint16_t *A, const uint
 // zero-padded to 128):
 //   H0 = x;  for l = 0, 1, 2:  X_l = [H_l | sum_{w in N(v)} H_l(w)]   (N x 256, bf16)
 //                               Z_l = X_l W_l^T + b_l                  (tensor cores, fp32)
-//                               H_{l+1} = relu(Z_l)
+//                               H_{l+1} = relu(Z_l)              (in the product's epilogue)
 //   y = (sum_v H_3(v)) . w_o + b_o        (predicted log(1 + cardinality))
 // trained with mean squared error and Adam, all on the device; the three
 // matrix products per layer of the forward and backward passes (X W^T,
@@ -89,11 +89,6 @@ __global__ void build_x(const float *__restrict__ H, const uint32_t *__restrict_
         X[(long long)v * kIn + f] = __float2bfloat16(H[i]);
         X[(long long)v * kIn + kH + f] = __float2bfloat16(s);
     }
-}
-
-__global__ void relu_copy(const float *__restrict__ Z, float *__restrict__ H, long long total) {
-    for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x)
-        H[i] = fmaxf(Z[i], 0.f);
 }
 
 // g[graph] = sum of H3 over the graph's nodes, in node order (deterministic);
@@ -121,16 +116,46 @@ __global__ void readout_out(const float *__restrict__ g, const float *__restrict
     if (lane == 0) y[warp] = s + bo[0];
 }
 
-// dy = 2 (y - t) / ng; loss += (y - t)^2 / ng; grads of w_o, b_o; dg = dy * w_o
-__global__ void loss_grad(const float *__restrict__ y, const float *__restrict__ t, const float *__restrict__ g,
-                          const float *__restrict__ wo, int ng, float *__restrict__ dy, float *__restrict__ loss,
-                          float *__restrict__ dwo, float *__restrict__ dbo) {
-    for (int G = blockIdx.x * blockDim.x + threadIdx.x; G < ng; G += gridDim.x * blockDim.x) {
-        const float r = y[G] - t[G];
-        dy[G] = 2.f * r / ng;
-        atomicAdd(loss, r * r / ng);
-        atomicAdd(dbo, dy[G]);
-        for (int f = 0; f < kH; ++f) atomicAdd(&dwo[f], dy[G] * g[(long long)G * kH + f]);
+// dy = 2 (y - t) / ng, loss = sum of (y - t)^2 / ng, db_o = sum of dy (block
+// kH); dw_o[f] = sum over G of dy[G] g[G][f] (block f).  Sums over a block in
+// a fixed order (an atomic per graph and feature on 128 addresses took 50 us).
+__global__ void __launch_bounds__(kT) loss_grad(const float *__restrict__ y, const float *__restrict__ t,
+                                                const float *__restrict__ g, int ng, float *__restrict__ dy,
+                                                float *__restrict__ loss, float *__restrict__ dwo,
+                                                float *__restrict__ dbo) {
+    __shared__ float red[2][kT / 32];
+    const int f = blockIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    float a = 0.f, b = 0.f;
+    for (int G = threadIdx.x; G < ng; G += kT) {
+        const float r = y[G] - t[G], d = 2.f * r / ng;
+        if (f < kH) {
+            a += d * g[(long long)G * kH + f];
+        } else {
+            dy[G] = d;
+            a += d;
+            b += r * r / ng;
+        }
+    }
+    for (int o = 16; o; o >>= 1) {
+        a += __shfl_xor_sync(0xffffffffu, a, o);
+        b += __shfl_xor_sync(0xffffffffu, b, o);
+    }
+    if (lane == 0) {
+        red[0][warp] = a;
+        red[1][warp] = b;
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        for (int w = 1; w < kT / 32; ++w) {
+            a += red[0][w];
+            b += red[1][w];
+        }
+        if (f < kH) {
+            dwo[f] = a;
+        } else {
+            *dbo = a;
+            *loss = b;
+        }
     }
 }
 
@@ -142,15 +167,15 @@ __global__ void readout_back(const float *__restrict__ dy, const float *__restri
         dH[i] = dy[gid[i / kH]] * wo[i % kH];
 }
 
-// dZ = dH * (Z > 0) as bf16; db += dZ (column sums)
-__global__ void relu_back(const float *__restrict__ dH, const float *__restrict__ Z, int n, __nv_bfloat16 *__restrict__ dZ,
+// dZ = dH * (Z > 0) as bf16, Z > 0 where relu(Z) is; db += dZ (column sums)
+__global__ void relu_back(const float *__restrict__ dH, const float *__restrict__ reluZ, int n, __nv_bfloat16 *__restrict__ dZ,
                           float *__restrict__ db) {
     __shared__ float part[kH];
     for (int f = threadIdx.x; f < kH; f += blockDim.x) part[f] = 0.f;
     __syncthreads();
     const long long total = (long long)n * kH;
     for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {
-        const float d = Z[i] > 0.f ? dH[i] : 0.f;
+        const float d = reluZ[i] > 0.f ? dH[i] : 0.f;
         dZ[i] = __float2bfloat16(d);
         atomicAdd(&part[i % kH], d);
     }
@@ -182,12 +207,12 @@ __global__ void adam(float *__restrict__ p, const float *__restrict__ gr, float 
     }
 }
 
-// x_in[v][f] = x[v][f] for f < F, 0 above (the first layer's width is 128)
-__global__ void pad_x(const float *__restrict__ x, uint32_t F, int n, float *__restrict__ x_in) {
+// H0[v][f] = x[v][f] for f < F, 0 above (the first layer's width is 128)
+__global__ void pad_x(const float *__restrict__ x, uint32_t F, int n, float *__restrict__ h0) {
     const long long total = (long long)n * kH;
     for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {
         const uint32_t f = (uint32_t)(i % kH);
-        x_in[i] = f < F ? x[(i / kH) * F + f] : 0.f;
+        h0[i] = f < F ? x[(i / kH) * F + f] : 0.f;
     }
 }
 
@@ -213,13 +238,20 @@ struct asdm_estimator {
     long long step = 0;
     // batch workspace (grown on demand)
     int cap_nodes = 0, cap_graphs = 0;
-    uint64_t cap_edges = 0;
-    float *x_stage = nullptr, *x_in = nullptr, *H = nullptr, *Z = nullptr, *dH = nullptr, *dX = nullptr, *gsum = nullptr, *y = nullptr,
-          *t = nullptr, *dy = nullptr, *loss = nullptr;
+    float *H = nullptr, *dH = nullptr, *dX = nullptr, *gsum = nullptr, *y = nullptr, *dy = nullptr, *loss = nullptr,
+          *part = nullptr;  // partial weight gradients (kMaxSplits products)
     __nv_bfloat16 *X = nullptr, *dZ = nullptr;
+    // the batch's inputs: the features, then everything else, assembled in
+    // in_host and uploaded in one copy (pinned memory would cost a new
+    // estimator's first batch 4 ms)
+    uint8_t *in = nullptr;
+    std::vector<uint8_t> in_host;
+    uint64_t cap_in = 0;
+    float *x_stage = nullptr, *t = nullptr;
     uint32_t *adj_off = nullptr, *adj = nullptr, *gid = nullptr;
     uint32_t *goff = nullptr, *gnodes = nullptr;  // nodes of each graph, ascending
 
+    static constexpr int kMaxSplits = 64;
     static constexpr long long kW = (long long)asdm::est::kH * asdm::est::kIn;
     float *W(int l) { return p + l * kW; }
     float *bias(int l) { return p + 3 * kW + l * asdm::est::kH; }
@@ -238,47 +270,40 @@ using namespace asdm::est;
 
 void free_batch(asdm_estimator *e) {
     cudaStream_t s = e->stream;
-    dfree(e->x_stage, s); dfree(e->x_in, s); dfree(e->H, s); dfree(e->Z, s); dfree(e->dH, s); dfree(e->dX, s); dfree(e->gsum, s);
-    dfree(e->y, s); dfree(e->t, s); dfree(e->dy, s); dfree(e->loss, s); dfree(e->X, s); dfree(e->dZ, s);
-    dfree(e->adj_off, s); dfree(e->adj, s); dfree(e->gid, s); dfree(e->goff, s); dfree(e->gnodes, s);
+    dfree(e->H, s); dfree(e->dH, s); dfree(e->dX, s); dfree(e->gsum, s); dfree(e->y, s); dfree(e->dy, s);
+    dfree(e->loss, s); dfree(e->X, s); dfree(e->dZ, s);
     e->cap_nodes = e->cap_graphs = 0;
-    e->cap_edges = 0;
 }
 
-int ensure_batch(asdm_estimator *e, int nodes, int graphs, uint64_t edges) {
-    if (nodes <= e->cap_nodes && graphs <= e->cap_graphs && edges <= e->cap_edges) return ASDM_OK;
-    free_batch(e);
+int ensure_batch(asdm_estimator *e, int nodes, int graphs, uint64_t in_bytes) {
     cudaStream_t s = e->stream;
+    if (in_bytes > e->cap_in) {
+        dfree(e->in, s);
+        e->cap_in = 0;
+        ASDM_TRY(dalloc(&e->in, in_bytes, s));
+        e->cap_in = in_bytes;
+    }
+    if (nodes <= e->cap_nodes && graphs <= e->cap_graphs) return ASDM_OK;
+    free_batch(e);
     const int N = std::max(nodes, 1), G = std::max(graphs, 1);
-    const uint64_t E = std::max<uint64_t>(edges, 1);
-    ASDM_TRY(dalloc(&e->x_stage, (uint64_t)N * e->in_features, s));
-    ASDM_TRY(dalloc(&e->x_in, (uint64_t)N * kH, s));
     ASDM_TRY(dalloc(&e->H, (uint64_t)(kLayers + 1) * N * kH, s));
-    ASDM_TRY(dalloc(&e->Z, (uint64_t)kLayers * N * kH, s));
     ASDM_TRY(dalloc(&e->dH, (uint64_t)N * kH, s));
     ASDM_TRY(dalloc(&e->dX, (uint64_t)N * kIn, s));
     ASDM_TRY(dalloc(&e->gsum, (uint64_t)G * kH, s));
     ASDM_TRY(dalloc(&e->y, G, s));
-    ASDM_TRY(dalloc(&e->t, G, s));
     ASDM_TRY(dalloc(&e->dy, G, s));
     ASDM_TRY(dalloc(&e->loss, 1, s));
     ASDM_TRY(dalloc(&e->X, (uint64_t)kLayers * N * kIn, s));
     ASDM_TRY(dalloc(&e->dZ, (uint64_t)N * kH, s));
-    ASDM_TRY(dalloc(&e->adj_off, (uint64_t)N + 1, s));
-    ASDM_TRY(dalloc(&e->adj, E, s));
-    ASDM_TRY(dalloc(&e->gid, N, s));
-    ASDM_TRY(dalloc(&e->goff, (uint64_t)G + 1, s));
-    ASDM_TRY(dalloc(&e->gnodes, N, s));
     e->cap_nodes = N;
     e->cap_graphs = G;
-    e->cap_edges = E;
     return ASDM_OK;
 }
 
 int gemm(asdm_estimator *e, tc::Operand A, tc::Operand B, int M, int N, int K, float *C, long long ldc,
-         const float *bias) {
-    dim3 grid((M + tc::kTileM - 1) / tc::kTileM, (N + tc::kTileN - 1) / tc::kTileN);
-    tc::gemm_kernel<<<grid, tc::kThreads, tc::kSmemBytes, e->stream>>>(A, B, M, N, K, C, ldc, bias, 0, e->err);
+         const float *bias, bool relu = false, int splits = 1) {
+    dim3 grid((M + tc::kTileM - 1) / tc::kTileM, (N + tc::kTileN - 1) / tc::kTileN, splits);
+    tc::gemm_kernel<<<grid, tc::kThreads, tc::kSmemBytes, e->stream>>>(A, B, M, N, K, C, ldc, bias, relu ? 1 : 0, e->err);
     ::asdm::count_launch();
     ASDM_CUDA(cudaGetLastError());
     return ASDM_OK;
@@ -288,17 +313,14 @@ int gemm(asdm_estimator *e, tc::Operand A, tc::Operand B, int M, int N, int K, f
 int forward(asdm_estimator *e, int n, int ng) {
     cudaStream_t s = e->stream;
     const long long nh = (long long)n * kH;
-    ASDM_CUDA(cudaMemcpyAsync(e->H, e->x_in, nh * sizeof(float), cudaMemcpyDeviceToDevice, s));
     for (int l = 0; l < kLayers; ++l) {
-        float *Hl = e->H + l * nh, *Hn = e->H + (l + 1) * nh, *Zl = e->Z + l * nh;
+        float *Hl = e->H + l * nh, *Hn = e->H + (l + 1) * nh;
         __nv_bfloat16 *Xl = e->X + (long long)l * n * kIn;
         build_x<<<grid_of(nh), kT, 0, s>>>(Hl, e->adj_off, e->adj, n, Xl);
         ::asdm::count_launch();
         tc::Operand a{Xl, kIn, 1, n};
         tc::Operand b{e->wb + l * asdm_estimator::kW, kIn, 1, kH};
-        ASDM_TRY(gemm(e, a, b, n, kH, kIn, Zl, kH, e->bias(l)));
-        relu_copy<<<grid_of(nh), kT, 0, s>>>(Zl, Hn, nh);
-        ::asdm::count_launch();
+        ASDM_TRY(gemm(e, a, b, n, kH, kIn, Hn, kH, e->bias(l), /*relu=*/true));
     }
     readout_sum<<<grid_of((long long)ng * kH), kT, 0, s>>>(e->H + kLayers * nh, e->goff, e->gnodes, ng, e->gsum);
     readout_out<<<(ng * 32 + kT - 1) / kT, kT, 0, s>>>(e->gsum, e->wo(), e->bo(), ng, e->y);
@@ -309,31 +331,51 @@ int forward(asdm_estimator *e, int n, int ng) {
 }
 
 int upload_batch(asdm_estimator *e, int n, int ng, const float *x, const uint32_t *adj_off, const uint32_t *adj,
-                 const uint32_t *node_graph) {
+                 const uint32_t *node_graph, const float *target) {
     const uint64_t ne = adj_off[n];
-    ASDM_TRY(ensure_batch(e, n, ng, ne));
-    cudaStream_t s = e->stream;
     for (int v = 0; v < n; ++v)
         if (node_graph[v] >= (uint32_t)ng) return fail(ASDM_ERR_INVALID, "node %d belongs to graph %u >= %d", v, node_graph[v], ng);
     for (uint64_t i = 0; i < ne; ++i)
         if (adj[i] >= (uint32_t)n) return fail(ASDM_ERR_INVALID, "adjacency entry out of range");
+    cudaStream_t s = e->stream;
+    // features; targets, adjacency, nodes by graph
+    uint64_t bytes = 0;
+    auto room = [&](uint64_t count) {
+        const uint64_t at = bytes;
+        bytes += (4 * count + 15) & ~15ull;
+        return at;
+    };
+    const uint64_t o_x = room((uint64_t)n * e->in_features), o_t = room(ng), o_off = room((uint64_t)n + 1), o_adj = room(ne),
+                   o_gid = room(n), o_goff = room((uint64_t)ng + 1), o_nodes = room(n);
+    ASDM_TRY(ensure_batch(e, n, ng, bytes));
+    e->in_host.resize(bytes - o_t);
+    uint8_t *h = e->in_host.data();
+    if (target) std::memcpy(h, target, (size_t)ng * 4);
+    std::memcpy(h + o_off - o_t, adj_off, ((size_t)n + 1) * 4);
+    if (ne) std::memcpy(h + o_adj - o_t, adj, ne * 4);
+    std::memcpy(h + o_gid - o_t, node_graph, (size_t)n * 4);
     // nodes grouped by graph (counting sort, stable)
-    std::vector<uint32_t> goff((size_t)ng + 1, 0), gnodes((size_t)n);
+    uint32_t *goff = reinterpret_cast<uint32_t *>(h + o_goff - o_t), *gnodes = reinterpret_cast<uint32_t *>(h + o_nodes - o_t);
+    std::memset(goff, 0, ((size_t)ng + 1) * 4);
     for (int v = 0; v < n; ++v) ++goff[node_graph[v] + 1];
     for (int G = 0; G < ng; ++G) goff[G + 1] += goff[G];
     {
-        std::vector<uint32_t> at(goff.begin(), goff.end() - 1);
+        std::vector<uint32_t> at(goff, goff + ng);
         for (int v = 0; v < n; ++v) gnodes[at[node_graph[v]]++] = (uint32_t)v;
     }
-    ASDM_CUDA(cudaMemcpyAsync(e->x_stage, x, (size_t)n * e->in_features * 4, cudaMemcpyHostToDevice, s));
-    pad_x<<<grid_of((long long)n * kH), kT, 0, s>>>(e->x_stage, e->in_features, n, e->x_in);
+    e->x_stage = reinterpret_cast<float *>(e->in + o_x);
+    e->t = reinterpret_cast<float *>(e->in + o_t);
+    e->adj_off = reinterpret_cast<uint32_t *>(e->in + o_off);
+    e->adj = reinterpret_cast<uint32_t *>(e->in + o_adj);
+    e->gid = reinterpret_cast<uint32_t *>(e->in + o_gid);
+    e->goff = reinterpret_cast<uint32_t *>(e->in + o_goff);
+    e->gnodes = reinterpret_cast<uint32_t *>(e->in + o_nodes);
+    // pageable sources: each call returns when its source has been read
+    ASDM_CUDA(cudaMemcpyAsync(e->in + o_x, x, (size_t)n * e->in_features * 4, cudaMemcpyHostToDevice, s));
+    ASDM_CUDA(cudaMemcpyAsync(e->in + o_t, h, bytes - o_t, cudaMemcpyHostToDevice, s));
+    pad_x<<<grid_of((long long)n * kH), kT, 0, s>>>(e->x_stage, e->in_features, n, e->H);
     ::asdm::count_launch();
-    ASDM_CUDA(cudaMemcpyAsync(e->adj_off, adj_off, (size_t)(n + 1) * 4, cudaMemcpyHostToDevice, s));
-    if (ne) ASDM_CUDA(cudaMemcpyAsync(e->adj, adj, ne * 4, cudaMemcpyHostToDevice, s));
-    ASDM_CUDA(cudaMemcpyAsync(e->gid, node_graph, (size_t)n * 4, cudaMemcpyHostToDevice, s));
-    ASDM_CUDA(cudaMemcpyAsync(e->goff, goff.data(), goff.size() * 4, cudaMemcpyHostToDevice, s));
-    ASDM_CUDA(cudaMemcpyAsync(e->gnodes, gnodes.data(), gnodes.size() * 4, cudaMemcpyHostToDevice, s));
-    ASDM_CUDA(cudaStreamSynchronize(s));  // host staging vectors go out of scope
+    ASDM_CUDA(cudaGetLastError());
     return ASDM_OK;
 }
 
@@ -364,6 +406,7 @@ extern "C" int asdm_est_create(uint32_t in_features, uint64_t seed, asdm_estimat
     ASDM_TRY(dalloc(&e->v, e->nparam, s));
     ASDM_TRY(dalloc(&e->wb, 3 * asdm_estimator::kW, s));
     ASDM_TRY(dalloc(&e->err, 1, s));
+    ASDM_TRY(dalloc(&e->part, (uint64_t)asdm_estimator::kMaxSplits * asdm_estimator::kW, s));
     // Xavier-uniform weights from a seeded generator, zero biases
     std::vector<float> hp(e->nparam, 0.f);
     Rng rng(seed);
@@ -387,7 +430,7 @@ extern "C" int asdm_est_predict(asdm_estimator *e, int n_nodes, int n_graphs, co
     clear_error();
     if (!e || !x || !adj_off || !node_graph || !out || n_nodes <= 0 || n_graphs <= 0)
         return fail(ASDM_ERR_INVALID, "bad estimator batch");
-    ASDM_TRY(upload_batch(e, n_nodes, n_graphs, x, adj_off, adj, node_graph));
+    ASDM_TRY(upload_batch(e, n_nodes, n_graphs, x, adj_off, adj, node_graph, nullptr));
     ASDM_TRY(forward(e, n_nodes, n_graphs));
     ASDM_CUDA(cudaMemcpyAsync(out, e->y, (size_t)n_graphs * 4, cudaMemcpyDeviceToHost, e->stream));
     return check_err(e);
@@ -399,27 +442,35 @@ extern "C" int asdm_est_train_step(asdm_estimator *e, int n_nodes, int n_graphs,
     clear_error();
     if (!e || !x || !adj_off || !node_graph || !target || n_nodes <= 0 || n_graphs <= 0)
         return fail(ASDM_ERR_INVALID, "bad estimator batch");
-    ASDM_TRY(upload_batch(e, n_nodes, n_graphs, x, adj_off, adj, node_graph));
+    ASDM_TRY(upload_batch(e, n_nodes, n_graphs, x, adj_off, adj, node_graph, target));
     cudaStream_t s = e->stream;
     const int n = n_nodes, ng = n_graphs;
     const long long nh = (long long)n * kH;
-    ASDM_CUDA(cudaMemcpyAsync(e->t, target, (size_t)ng * 4, cudaMemcpyHostToDevice, s));
     ASDM_TRY(forward(e, n, ng));
-    ASDM_CUDA(cudaMemsetAsync(e->g, 0, e->nparam * 4, s));
-    ASDM_CUDA(cudaMemsetAsync(e->loss, 0, 4, s));
-    loss_grad<<<grid_of(ng), kT, 0, s>>>(e->y, e->t, e->gsum, e->wo(), ng, e->dy, e->loss, e->gwo(), e->gbo());
+    // the bias gradients are added up by atomics; every other gradient is written
+    ASDM_CUDA(cudaMemsetAsync(e->gbias(0), 0, kLayers * kH * 4, s));
+    loss_grad<<<kH + 1, kT, 0, s>>>(e->y, e->t, e->gsum, ng, e->dy, e->loss, e->gwo(), e->gbo());
     readout_back<<<grid_of(nh), kT, 0, s>>>(e->dy, e->wo(), e->gid, n, e->dH);
     ::asdm::count_launch();
     ::asdm::count_launch();
     for (int l = kLayers - 1; l >= 0; --l) {
-        float *Zl = e->Z + l * nh;
         __nv_bfloat16 *Xl = e->X + (long long)l * n * kIn;
-        relu_back<<<grid_of(nh), kT, 0, s>>>(e->dH, Zl, n, e->dZ, e->gbias(l));
+        relu_back<<<grid_of(nh), kT, 0, s>>>(e->dH, e->H + (l + 1) * nh, n, e->dZ, e->gbias(l));
         ::asdm::count_launch();
         // dW_l[o][i] = sum_v dZ[v][o] X_l[v][i]   (M = 128 outputs, N = 256 inputs, K = nodes)
         tc::Operand a{e->dZ, 1, kH, kH};
         tc::Operand b{Xl, 1, kIn, kIn};
-        ASDM_TRY(gemm(e, a, b, kH, kIn, n, e->gW(l), kIn, nullptr));
+        // in splits of at least two chunks of nodes
+        const int chunks = (n + tc::kChunkK - 1) / tc::kChunkK;
+        const int per = (chunks + asdm_estimator::kMaxSplits - 1) / asdm_estimator::kMaxSplits;
+        const int splits = (chunks + std::max(per, 2) - 1) / std::max(per, 2);  // none is empty
+        if (splits == 1) {
+            ASDM_TRY(gemm(e, a, b, kH, kIn, n, e->gW(l), kIn, nullptr));
+        } else {
+            ASDM_TRY(gemm(e, a, b, kH, kIn, n, e->part, kIn, nullptr, false, splits));
+            tc::split_sum<<<grid_of(asdm_estimator::kW), kT, 0, s>>>(e->part, splits, asdm_estimator::kW, e->gW(l));
+            ::asdm::count_launch();
+        }
         if (l > 0) {
             // dX_l[v][i] = sum_o dZ[v][o] W_l[o][i]   (M = nodes, N = 256, K = 128)
             tc::Operand a2{e->dZ, kH, 1, n};
@@ -467,6 +518,8 @@ extern "C" void asdm_est_free(asdm_estimator *e) {
     if (!e) return;
     free_batch(e);
     cudaStream_t s = e->stream;
+    dfree(e->in, s);
+    dfree(e->part, s);
     dfree(e->p, s); dfree(e->g, s); dfree(e->m, s); dfree(e->v, s); dfree(e->wb, s); dfree(e->err, s);
     cudaStreamSynchronize(s);
     cudaStreamDestroy(s);

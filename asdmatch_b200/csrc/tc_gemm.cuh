@@ -2,15 +2,24 @@
 //
 //   D[m][n] = sum_k A(m, k) * B(n, k)      one 128 x 128 output tile per CTA
 //
-// A and B are read from global memory through caller-supplied strides (so a
-// transposed operand costs nothing extra), staged 64 K-elements at a time into
-// shared memory in the canonical K-major, no-swizzle core-matrix layout
-// (8 rows x 16 bytes per core matrix), and multiplied by tcgen05.mma issued
-// from one thread, M=128 N=128 K=16 per instruction, accumulating in tensor
-// memory.  tcgen05.commit arrives on an mbarrier that every thread waits on
-// (bounded) before the shared buffers are refilled or the accumulator is read
-// back with tcgen05.ld.  128 threads (4 warps): warp w owns TMEM lanes
-// 32w..32w+31, i.e. output rows 32w..32w+31 of the tile.
+// A and B are read from global memory through caller-supplied strides, 64
+// K-elements at a time, into shared memory in the canonical K-major,
+// no-swizzle core-matrix layout (8 rows x 16 bytes per core matrix), and
+// multiplied by tcgen05.mma issued from one thread, M=128 N=128 K=16 per
+// instruction, accumulating in tensor memory.  An operand whose K runs along
+// memory is copied with 16-byte cp.async, one whose rows do is loaded 16 bytes
+// at a time and transposed in registers, 8 x 8 elements a thread; element by
+// element only where alignment or a ragged edge asks for it.  kStages chunks
+// of shared memory are in rotation: chunks are fetched kStages - 1 ahead of
+// the tensor cores (element-wise, unbuffered staging took 10 us a chunk: a
+// forward product of 4,600 nodes 97 us).  With splits, the K chunks are
+// divided among grid.z CTAs, whose fp32 partial products split_sum adds in
+// order: the weight gradients' K is the node count, which would otherwise
+// leave two CTAs working.
+// tcgen05.commit arrives on the stage's mbarrier, waited for (bounded) before
+// the stage is refilled or the accumulator is read back with tcgen05.ld.
+// 128 threads (4 warps): warp w owns TMEM lanes 32w..32w+31, i.e. output rows
+// 32w..32w+31 of the tile.
 #pragma once
 
 #include <cuda_bf16.h>
@@ -23,11 +32,14 @@ constexpr int kTileM = 128, kTileN = 128, kChunkK = 64;
 constexpr int kThreads = 128;
 constexpr uint32_t kTmemCols = 128;
 constexpr uint32_t kWaitSpins = 1u << 22;
-// shared memory: A chunk + B chunk (16 KB each), mbarrier, TMEM address.
-// Requested at 72 KB so that at most 3 CTAs share an SM: 3 x 128 TMEM
+constexpr int kStages = 3;
+// Core matrices lie kCore bytes apart along the rows (16 more than their 128,
+// so that stores of one row of neighbouring matrices fall into different
+// banks) and kGroup apart along K.
+constexpr int kCore = 144, kGroup = (kTileM / 8) * kCore, kOperand = (kChunkK / 8) * kGroup;
+// stages, mbarriers, TMEM address.  At most two CTAs share an SM: 2 x 128 TMEM
 // columns never exceed the SM's 512, so tcgen05.alloc never has to wait.
-constexpr int kSmemUsed = 2 * kTileM * kChunkK * 2 + 64;
-constexpr int kSmemBytes = 72 * 1024;
+constexpr int kSmemBytes = kStages * 2 * kOperand + 64;
 
 // Operand view: element (r, k) at ptr[r * sr + k * sk]; rows >= rows_valid
 // and k >= K read as zero.
@@ -56,30 +68,85 @@ __host__ __device__ constexpr uint32_t idesc_bf16_f32() {
     return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(kTileN >> 3) << 17) | ((uint32_t)(kTileM >> 4) << 24);
 }
 
-// Stage rows [r0, r0+128) x k [k0, k0+64) of an operand into the core-matrix
-// layout: core (row group g, k group c) at byte ((c * 16) + g) * 128, row r of
-// the group at +16 r, 8 bf16 per row.
-__device__ __forceinline__ void stage(__nv_bfloat16 *dst, const Operand &op, int r0, int k0, int K) {
-    for (int i = threadIdx.x; i < kTileM * kChunkK; i += kThreads) {
-        const int r = i / kChunkK, k = i % kChunkK;
+// Byte offset of element (row r, k) of a staged chunk: core (row group, k
+// group) at kGroup * (k / 8) + kCore * (r / 8), row r of the group at +16 r.
+__device__ __forceinline__ int staged_at(int r, int k) { return (k >> 3) * kGroup + (r >> 3) * kCore + (r & 7) * 16 + (k & 7) * 2; }
+
+__device__ __forceinline__ void stage_core_row(uint8_t *dst, const Operand &op, int gr, int gk, int K) {
+    __nv_bfloat16 *d = reinterpret_cast<__nv_bfloat16 *>(dst);
+#pragma unroll
+    for (int j = 0; j < 8; ++j)
+        d[j] = gr < op.rows_valid && gk + j < K ? op.ptr[(long long)gr * op.sr + (long long)(gk + j) * op.sk]
+                                                : __float2bfloat16(0.f);
+}
+
+// Stage rows [r0, r0+128) x k [k0, k0+64) of an operand.
+__device__ __forceinline__ void stage(uint8_t *dst, const Operand &op, int r0, int k0, int K) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    if (op.sr == 1 && op.sk % 8 == 0 && (reinterpret_cast<uintptr_t>(op.ptr) & 15) == 0) {
+        // rows along memory: thread (k group, row group) loads 8 rows of 8 k and transposes them
+        const int rg = threadIdx.x & 15, kg = threadIdx.x >> 4, gr = r0 + 8 * rg, gk = k0 + 8 * kg;
+        uint8_t *d = dst + kg * kGroup + rg * kCore;
+        if (gr + 8 <= op.rows_valid) {
+            uint32_t w[8][4];
+#pragma unroll
+            for (int j = 0; j < 8; ++j) {
+                uint4 v = make_uint4(0, 0, 0, 0);
+                if (gk + j < K) v = *reinterpret_cast<const uint4 *>(op.ptr + gr + (long long)(gk + j) * op.sk);
+                w[j][0] = v.x; w[j][1] = v.y; w[j][2] = v.z; w[j][3] = v.w;
+            }
+#pragma unroll
+            for (int r = 0; r < 8; ++r) {
+                uint32_t o[4];
+#pragma unroll
+                for (int j = 0; j < 4; ++j)  // k 2j and 2j + 1 of row r
+                    o[j] = __byte_perm(w[2 * j][r >> 1], w[2 * j + 1][r >> 1], (r & 1) ? 0x7632 : 0x5410);
+                *reinterpret_cast<uint4 *>(d + 16 * r) = make_uint4(o[0], o[1], o[2], o[3]);
+            }
+        } else {
+            for (int r = 0; r < 8; ++r) stage_core_row(d + 16 * r, op, gr + r, gk, K);
+        }
+        return;
+    }
+    const bool vec = op.sk == 1 && op.sr % 8 == 0 && (reinterpret_cast<uintptr_t>(op.ptr) & 15) == 0;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+        // a warp copies 8 rows x 4 k groups: whole core matrices
+        const int c = i * 4 + warp, r = (c >> 1) * 8 + (lane & 7), k = ((c & 1) * 4 + (lane >> 3)) * 8;
+        uint8_t *d = dst + staged_at(r, k);
         const int gr = r0 + r, gk = k0 + k;
-        __nv_bfloat16 v = __float2bfloat16(0.f);
-        if (gr < op.rows_valid && gk < K) v = op.ptr[(long long)gr * op.sr + (long long)gk * op.sk];
-        const int off = (((k >> 3) * (kTileM / 8) + (r >> 3)) * 64) + ((r & 7) * 8) + (k & 7);  // in elements
-        dst[off] = v;
+        const bool in = gr < op.rows_valid && gk < K;
+        if (vec && (!in || gk + 8 <= K)) {
+            const __nv_bfloat16 *src = in ? op.ptr + (long long)gr * op.sr + gk : op.ptr;
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(smem_u32(d)), "l"(src), "r"(in ? 16 : 0));
+        } else {
+            stage_core_row(d, op, gr, gk, K);
+        }
     }
 }
 
-// Computes one 128x128 tile into acc_out (fp32, row-major with stride ldc),
-// rows >= m_valid / cols >= n_valid not written.  `err` gets 1 if a wait on
+// Waits (bounded) for the mbarrier's phase.
+__device__ __forceinline__ bool wait_phase(uint64_t *mbar, uint32_t parity) {
+    uint32_t done = 0;
+    for (uint32_t it = 0; it < kWaitSpins && !done; ++it) {
+        asm volatile(
+            "{\n\t.reg .pred p;\n\t"
+            "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+            "selp.u32 %0, 1, 0, p;\n\t}\n"
+            : "=r"(done)
+            : "r"(smem_u32(mbar)), "r"(parity));
+    }
+    return done != 0;
+}
+
+// Computes one 128x128 tile of the K chunks [c0, c1) into C (fp32, row-major
+// with stride ldc), rows >= m_valid / cols >= n_valid not written.  `err` gets 1 if a wait on
 // the tensor cores ran out of its bound (the tile is then not written).
-__device__ void gemm_tile(const Operand &A, const Operand &B, int K, int m0, int n0, float *C, long long ldc,
-                          int m_valid, int n_valid, const float *bias, bool relu, unsigned int *err) {
+__device__ void gemm_tile(const Operand &A, const Operand &B, int K, int c0, int c1, int m0, int n0, float *C,
+                          long long ldc, int m_valid, int n_valid, const float *bias, bool relu, unsigned int *err) {
     extern __shared__ __align__(1024) uint8_t smem[];
-    __nv_bfloat16 *sA = reinterpret_cast<__nv_bfloat16 *>(smem);
-    __nv_bfloat16 *sB = sA + kTileM * kChunkK;
-    uint64_t *mbar = reinterpret_cast<uint64_t *>(smem + 2 * kTileM * kChunkK * 2);
-    uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(mbar + 1);
+    uint64_t *mbar = reinterpret_cast<uint64_t *>(smem + kStages * 2 * kOperand);
+    uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(mbar + kStages);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
 
     if (warp == 0) {
@@ -87,30 +154,38 @@ __device__ void gemm_tile(const Operand &A, const Operand &B, int K, int m0, int
                      "r"(kTmemCols));
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
     }
-    if (threadIdx.x == 0) {
-        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(mbar)));
-    }
+    if (threadIdx.x < kStages) asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(mbar + threadIdx.x)));
     asm volatile("tcgen05.fence::before_thread_sync;");
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;");
     const uint32_t tmem = *tmem_slot;
 
     bool ok = true;
-    uint32_t phase = 0;
+    const int nc = c1 - c0;
     const uint32_t idesc = idesc_bf16_f32();
-    for (int k0 = 0; k0 < K && ok; k0 += kChunkK) {
-        stage(sA, A, m0, k0, K);
-        stage(sB, B, n0, k0, K);
+    auto fetch = [&](int i) {  // chunk i of this CTA into its stage (an empty group past the end)
+        if (i < nc) {
+            uint8_t *d = smem + (i % kStages) * 2 * kOperand;
+            stage(d, A, m0, (c0 + i) * kChunkK, K);
+            stage(d + kOperand, B, n0, (c0 + i) * kChunkK, K);
+        }
+        asm volatile("cp.async.commit_group;");
+    };
+#pragma unroll
+    for (int i = 0; i < kStages - 1; ++i) fetch(i);
+    for (int i = 0; i < nc && ok; ++i) {
+        asm volatile("cp.async.wait_group %0;" ::"n"(kStages - 2));  // chunk i has landed
         // make the generic-proxy smem writes visible to the tensor cores
         asm volatile("fence.proxy.async.shared::cta;");
         __syncthreads();
         if (threadIdx.x == 0) {
             asm volatile("tcgen05.fence::after_thread_sync;");
+            const uint32_t sa = smem_u32(smem + (i % kStages) * 2 * kOperand), sb = sa + kOperand;
             for (int s = 0; s < kChunkK / 16; ++s) {
-                // K slice s: k groups 2s, 2s+1 -> byte offset 2s * 16 * 128
-                const uint64_t da = make_desc(smem_u32(sA) + s * 2 * (kTileM / 8) * 128, (kTileM / 8) * 128, 128);
-                const uint64_t db = make_desc(smem_u32(sB) + s * 2 * (kTileN / 8) * 128, (kTileN / 8) * 128, 128);
-                const uint32_t accumulate = (k0 > 0 || s > 0) ? 1u : 0u;
+                // K slice s: k groups 2s, 2s+1
+                const uint64_t da = make_desc(sa + s * 2 * kGroup, kGroup, kCore);
+                const uint64_t db = make_desc(sb + s * 2 * kGroup, kGroup, kCore);
+                const uint32_t accumulate = (i > 0 || s > 0) ? 1u : 0u;
                 asm volatile(
                     "{\n\t.reg .pred p;\n\t"
                     "setp.ne.b32 p, %4, 0;\n\t"
@@ -119,21 +194,17 @@ __device__ void gemm_tile(const Operand &A, const Operand &B, int K, int m0, int
                     : "r"(tmem), "l"(da), "l"(db), "r"(idesc), "r"(accumulate), "r"(0u), "r"(0u), "r"(0u), "r"(0u));
             }
             asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
-                smem_u32(mbar)));
+                smem_u32(mbar + i % kStages)));
         }
-        // every thread waits for the MMAs before the buffers are reused
-        uint32_t done = 0;
-        for (uint32_t it = 0; it < kWaitSpins && !done; ++it) {
-            asm volatile(
-                "{\n\t.reg .pred p;\n\t"
-                "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-                "selp.u32 %0, 1, 0, p;\n\t}\n"
-                : "=r"(done)
-                : "r"(smem_u32(mbar)), "r"(phase));
-        }
-        ok = __syncthreads_and(done != 0);
-        phase ^= 1;
+        // the next fetch goes into the stage that chunk i - 1 was read from
+        bool done = true;
+        if (i > 0) done = wait_phase(mbar + (i - 1) % kStages, (uint32_t)((i - 1) / kStages) & 1u);
+        ok = __syncthreads_and(done);
+        if (ok) fetch(i + kStages - 1);
     }
+    asm volatile("cp.async.wait_all;");
+    // the last chunk's products (its commit covers all before it)
+    if (nc > 0) ok = __syncthreads_and(ok && wait_phase(mbar + (nc - 1) % kStages, (uint32_t)((nc - 1) / kStages) & 1u));
     asm volatile("tcgen05.fence::after_thread_sync;");
     if (ok) {
         const int row = m0 + warp * 32 + lane;
@@ -148,7 +219,7 @@ __device__ void gemm_tile(const Operand &A, const Operand &B, int K, int m0, int
                 for (int j = 0; j < 8; ++j) {
                     const int col = n0 + c + j;
                     if (col < n_valid) {
-                        float v = __uint_as_float(r[j]);
+                        float v = nc > 0 ? __uint_as_float(r[j]) : 0.f;  // no chunks: nothing was accumulated
                         if (bias) v += bias[col];
                         if (relu) v = fmaxf(v, 0.f);
                         C[(long long)row * ldc + col] = v;
@@ -157,17 +228,7 @@ __device__ void gemm_tile(const Operand &A, const Operand &B, int K, int m0, int
             }
         }
     } else {
-        // a wait ran out: give any MMA still in flight one more bounded wait
-        // before the accumulator's tensor memory is released
-        uint32_t done = 0;
-        for (uint32_t it = 0; it < kWaitSpins && !done; ++it) {
-            asm volatile(
-                "{\n\t.reg .pred p;\n\t"
-                "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-                "selp.u32 %0, 1, 0, p;\n\t}\n"
-                : "=r"(done)
-                : "r"(smem_u32(mbar)), "r"(phase ^ 1u));
-        }
+        // a wait ran out (each was bounded; the last one covered every MMA in flight)
         if (threadIdx.x == 0) atomicExch(err, 1u);
     }
     asm volatile("tcgen05.fence::before_thread_sync;");
@@ -175,10 +236,24 @@ __device__ void gemm_tile(const Operand &A, const Operand &B, int K, int m0, int
     if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(kTmemCols));
 }
 
-// grid (ceil(M/128), ceil(N/128)); dynamic shared memory kSmemBytes.
+// grid (ceil(M/128), ceil(N/128), splits); dynamic shared memory kSmemBytes.
+// With splits > 1, split z writes its partial product to C + z * M * ldc.
 __global__ void __launch_bounds__(kThreads) gemm_kernel(Operand A, Operand B, int M, int N, int K, float *C, long long ldc,
                                                         const float *bias, int relu, unsigned int *err) {
-    gemm_tile(A, B, K, blockIdx.x * kTileM, blockIdx.y * kTileN, C, ldc, M, N, bias, relu != 0, err);
+    const int chunks = (K + kChunkK - 1) / kChunkK, per = (chunks + (int)gridDim.z - 1) / (int)gridDim.z;
+    const int c0 = min(chunks, (int)blockIdx.z * per), c1 = min(chunks, c0 + per);
+    gemm_tile(A, B, K, c0, c1, blockIdx.x * kTileM, blockIdx.y * kTileN, C + (long long)blockIdx.z * M * ldc, ldc, M, N,
+              bias, relu != 0, err);
+}
+
+// out[i] = sum of the splits' partial products, in order.
+__global__ void split_sum(const float *__restrict__ part, int splits, long long n, float *__restrict__ out) {
+    for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
+        float s = 0.f;
+#pragma unroll 8
+        for (int z = 0; z < splits; ++z) s += part[z * n + i];
+        out[i] = s;
+    }
 }
 
 }  // namespace tc
