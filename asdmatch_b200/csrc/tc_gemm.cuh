@@ -208,22 +208,33 @@ __device__ void gemm_tile(const Operand &A, const Operand &B, int K, int c0, int
     asm volatile("tcgen05.fence::after_thread_sync;");
     if (ok) {
         const int row = m0 + warp * 32 + lane;
-        for (int c = 0; c < kTileN; c += 8) {
-            uint32_t r[8];
-            asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];\n"
-                         : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
+        const bool vec = (ldc & 3) == 0 && (n_valid & 3) == 0 && (reinterpret_cast<uintptr_t>(C) & 15) == 0;
+        for (int c = 0; c < kTileN; c += 16) {
+            uint32_t r[16];
+            asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, "
+                         "%14, %15}, [%16];\n"
+                         : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
+                           "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
                          : "r"(tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)c));
             asm volatile("tcgen05.wait::ld.sync.aligned;");
-            if (row < m_valid) {
+            if (row >= m_valid) continue;
 #pragma unroll
-                for (int j = 0; j < 8; ++j) {
-                    const int col = n0 + c + j;
-                    if (col < n_valid) {
-                        float v = nc > 0 ? __uint_as_float(r[j]) : 0.f;  // no chunks: nothing was accumulated
-                        if (bias) v += bias[col];
-                        if (relu) v = fmaxf(v, 0.f);
-                        C[(long long)row * ldc + col] = v;
-                    }
+            for (int j = 0; j < 16; j += 4) {
+                const int col = n0 + c + j;
+                float v[4];
+#pragma unroll
+                for (int t = 0; t < 4; ++t) {
+                    v[t] = nc > 0 ? __uint_as_float(r[j + t]) : 0.f;  // no chunks: nothing was accumulated
+                    if (bias && col + t < n_valid) v[t] += bias[col + t];
+                    if (relu) v[t] = fmaxf(v[t], 0.f);
+                }
+                float *dst = C + (long long)row * ldc + col;
+                if (vec && col < n_valid) {
+                    *reinterpret_cast<float4 *>(dst) = make_float4(v[0], v[1], v[2], v[3]);
+                } else {
+#pragma unroll
+                    for (int t = 0; t < 4; ++t)
+                        if (col + t < n_valid) dst[t] = v[t];
                 }
             }
         }
