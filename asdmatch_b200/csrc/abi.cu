@@ -6,6 +6,7 @@
 #include <new>
 
 #include "cs.cuh"
+#include "local.cuh"
 
 namespace asdm {
 namespace {
@@ -352,10 +353,10 @@ int build_prefix_plan(const asdm_cs &cs, const uint32_t *order, uint32_t depth, 
 int run_batch_count(asdm_graph *G, const std::vector<asdm_cs *> &cs, const std::vector<const asdm_plan *> &plans,
                     double time_limit_s, uint64_t count_limit, uint64_t *counts, int *status, asdm_run_stats *agg,
                     uint64_t *const *local_out, uint64_t *cycles = nullptr, double query_time_s = 0.0,
-                    bool settled = false);
+                    bool settled = false, HostFill *fill = nullptr);
 int settle_queries(asdm_graph *G, const std::vector<asdm_cs *> &cs, const std::vector<char> &full,
                    std::vector<uint32_t> &live, uint64_t count_limit, uint64_t *counts, int *status,
-                   asdm_run_stats *agg, uint64_t *const *local_out);
+                   asdm_run_stats *agg, uint64_t *const *local_out, HostFill *fill = nullptr);
 int plan_batch_learned(const std::vector<asdm_cs *> &css, asdm_estimator *e, uint32_t kmax,
                        std::vector<asdm_plan> &plans);
 }  // namespace asdm
@@ -377,6 +378,7 @@ static int run_batch_impl(asdm_graph *g, uint32_t nq, const uint32_t *q_sizes, c
         return fail(ASDM_ERR_INVALID, "null argument");
     std::vector<std::unique_ptr<asdm_cs>> all(nq);
     std::vector<uint64_t> state(nq, 0);
+    std::vector<std::pair<uint64_t *, uint64_t>> outs;  // the caller's local-count matrices
     for (uint32_t i = 0; i < nq; ++i) {
         counts[i] = 0;
         status[i] = ASDM_OK;
@@ -394,10 +396,12 @@ static int run_batch_impl(asdm_graph *g, uint32_t nq, const uint32_t *q_sizes, c
         }
         if (local_out) {
             state[i] += 8ull * g->d.n * c->q.n;  // the query's local-count block
-            if (local_out[i]) std::fill(local_out[i], local_out[i] + (uint64_t)g->d.n * c->q.n, 0ull);
+            if (local_out[i]) outs.emplace_back(local_out[i], (uint64_t)g->d.n * c->q.n);
         }
         all[i] = std::move(c);
     }
+    HostFill fill;  // zeroed meanwhile (the matrices of queries without a result stay zero)
+    fill.start(outs);
     int worst = ASDM_OK;
     for (uint32_t i = 0; i < nq && worst != ASDM_ERR_CUDA; ++i)
         if (status[i] != ASDM_OK && worst == ASDM_OK) worst = status[i];
@@ -438,7 +442,7 @@ static int run_batch_impl(asdm_graph *g, uint32_t nq, const uint32_t *q_sizes, c
                 for (uint32_t id : ids) slo.push_back(local_out[id]);
             const std::vector<uint32_t> before = live;
             rc = settle_queries(g, group, full, live, count_limit, sc.data(), sst.data(), &gs,
-                                local_out ? slo.data() : nullptr);
+                                local_out ? slo.data() : nullptr, &fill);
             if (rc != ASDM_OK) {
                 for (uint32_t id : ids) status[id] = rc;
                 if (worst == ASDM_OK) worst = rc;
@@ -487,7 +491,7 @@ static int run_batch_impl(asdm_graph *g, uint32_t nq, const uint32_t *q_sizes, c
         {
             asdm_run_stats es{};
             rc = run_batch_count(g, run_cs, run_plans, time_limit_s, count_limit, c.data(), st.data(), &es,
-                                 local_out ? lo.data() : nullptr, nullptr, query_time_s, /*settled=*/true);
+                                 local_out ? lo.data() : nullptr, nullptr, query_time_s, /*settled=*/true, &fill);
             gs.count += es.count;
             gs.intersections += es.intersections;
             gs.list_bytes += es.list_bytes;

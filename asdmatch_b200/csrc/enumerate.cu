@@ -28,6 +28,7 @@
 #include <mutex>
 
 #include "cs.cuh"
+#include "local.cuh"
 #include "rows.cuh"
 
 namespace asdm {
@@ -1869,8 +1870,8 @@ int run_plan(asdm_cs &cs, const asdm_plan &plan, const asdm_run_opts &opt, asdm_
     const uint32_t n = q.n;
     const uint32_t mode = opt.mode & (ASDM_MODE_LOCAL | ASDM_MODE_EMBED);
     st = asdm_run_stats{};
-    if (opt.local_counts && (mode & ASDM_MODE_LOCAL))
-        std::fill(opt.local_counts, opt.local_counts + (uint64_t)G->d.n * n, 0ull);
+    HostFill fill;
+    if (opt.local_counts && (mode & ASDM_MODE_LOCAL)) fill.start({{opt.local_counts, (uint64_t)G->d.n * n}});
     if (!cs.nonempty) return ASDM_OK;
     if (mode == ASDM_MODE_LOCAL && opt.local_counts && plan.order.size() == n && tree_countable(q)) {
         // conflict-free tree: counts and local counts from the tree program
@@ -1893,11 +1894,7 @@ int run_plan(asdm_cs &cs, const asdm_plan &plan, const asdm_run_opts &opt, asdm_
         cudaEventElapsedTime(&tms, t0, t1);
         cudaEventDestroy(t0);
         cudaEventDestroy(t1);
-        if (trc == ASDM_OK && done[0] &&
-            (cudaMemcpyAsync(opt.local_counts, blk, local_n * sizeof(unsigned long long), cudaMemcpyDeviceToHost, s) !=
-                 cudaSuccess ||
-             cudaStreamSynchronize(s) != cudaSuccess))
-            trc = fail(ASDM_ERR_CUDA, "local-count readback failed");
+        if (trc == ASDM_OK && done[0]) trc = read_locals(G, {LocalRead{&cs, blk, opt.local_counts}}, fill);
         dfree(blk, s);
         cudaStreamSynchronize(s);
         if (trc != ASDM_OK) return trc;
@@ -2089,14 +2086,9 @@ int run_plan(asdm_cs &cs, const asdm_plan &plan, const asdm_run_opts &opt, asdm_
         if (flags & kFlagTimeout) { rc = fail(ASDM_ERR_TIMEOUT, "time limit reached"); break; }
         if (flags & kFlagLimit) { rc = fail(ASDM_ERR_LIMIT, "count limit reached"); break; }
         if (a.lw && (rc = push_leaf_weights({&cs}, {&plan}, {a.lw}, {d_local}, G->num_sms, s))) break;
-        if ((mode & ASDM_MODE_LOCAL) && opt.local_counts) {
-            if (cudaMemcpyAsync(opt.local_counts, d_local, local_n * sizeof(unsigned long long), cudaMemcpyDeviceToHost,
-                                s) != cudaSuccess ||
-                cudaStreamSynchronize(s) != cudaSuccess) {
-                rc = fail(ASDM_ERR_CUDA, "local-count readback failed");
-                break;
-            }
-        }
+        if ((mode & ASDM_MODE_LOCAL) && opt.local_counts &&
+            (rc = read_locals(G, {LocalRead{&cs, d_local, opt.local_counts}}, fill)))
+            break;
         if (mode & ASDM_MODE_EMBED) {
             const uint64_t rows = ctr[kCtrRows];
             st.emb_rows = std::min<uint64_t>(rows, row_cap);
@@ -2127,7 +2119,7 @@ int run_plan(asdm_cs &cs, const asdm_plan &plan, const asdm_run_opts &opt, asdm_
 // the settled ones are written, their device time is added to agg->kernel_ms.
 int settle_queries(asdm_graph *G, const std::vector<asdm_cs *> &cs, const std::vector<char> &full,
                    std::vector<uint32_t> &live, uint64_t count_limit, uint64_t *counts, int *status,
-                   asdm_run_stats *agg, uint64_t *const *local_out) {
+                   asdm_run_stats *agg, uint64_t *const *local_out, HostFill *fill) {
     cudaStream_t s = G->stream;
     const uint32_t Q = (uint32_t)cs.size();
     if (live.empty()) return ASDM_OK;
@@ -2167,13 +2159,13 @@ int settle_queries(asdm_graph *G, const std::vector<asdm_cs *> &cs, const std::v
             trc = cudaMemsetAsync(blk, 0, words * sizeof(unsigned long long), s) == cudaSuccess
                       ? tree_counts(G, tcs, tc, done, &blocks)
                       : fail(ASDM_ERR_CUDA, "local-count reset failed");
+            std::vector<LocalRead> reads;
+            for (size_t k = 0; k < ids.size() && trc == ASDM_OK; ++k)
+                if (done[k] && local_out[ids[k]]) reads.push_back(LocalRead{cs[ids[k]], blocks[k], local_out[ids[k]]});
+            if (!reads.empty()) trc = read_locals(G, reads, *fill);
             for (size_t k = 0; k < ids.size() && trc == ASDM_OK; ++k) {
                 if (!done[k]) continue;
                 const uint32_t i = ids[k];
-                if (local_out[i] &&
-                    cudaMemcpyAsync(local_out[i], blocks[k], (uint64_t)G->d.n * cs[i]->q.n * sizeof(unsigned long long),
-                                    cudaMemcpyDeviceToHost, s) != cudaSuccess)
-                    trc = fail(ASDM_ERR_CUDA, "local-count readback failed");
                 settled[i] = 1;
                 counts[i] = tc[k];
                 if (count_limit && tc[k] > count_limit) status[i] = ASDM_ERR_LIMIT;
@@ -2279,7 +2271,7 @@ int settle_queries(asdm_graph *G, const std::vector<asdm_cs *> &cs, const std::v
 
 int run_batch_count(asdm_graph *G, const std::vector<asdm_cs *> &cs, const std::vector<const asdm_plan *> &plans,
                     double time_limit_s, uint64_t count_limit, uint64_t *counts, int *status, asdm_run_stats *agg,
-                    uint64_t *const *local_out, uint64_t *cycles, double query_time_s, bool settled) {
+                    uint64_t *const *local_out, uint64_t *cycles, double query_time_s, bool settled, HostFill *fill) {
     cudaStream_t s = G->stream;
     const uint32_t Q = (uint32_t)cs.size();
     std::vector<uint32_t> live;  // queries with a non-empty candidate space
@@ -2294,7 +2286,7 @@ int run_batch_count(asdm_graph *G, const std::vector<asdm_cs *> &cs, const std::
     if (!settled) {
         std::vector<char> full(Q, 0);
         for (uint32_t i = 0; i < Q; ++i) full[i] = plans[i]->order.size() == cs[i]->q.n;
-        ASDM_TRY(settle_queries(G, cs, full, live, count_limit, counts, status, agg, local_out));
+        ASDM_TRY(settle_queries(G, cs, full, live, count_limit, counts, status, agg, local_out, fill));
         if (live.empty()) return ASDM_OK;
     }
     const uint32_t L = (uint32_t)live.size();
@@ -2545,13 +2537,10 @@ int run_batch_count(asdm_graph *G, const std::vector<asdm_cs *> &cs, const std::
             rc = push_leaf_weights(tcs, tpl, lwv, blocks, G->num_sms, s);
         }
         if (rc == ASDM_OK && local_mode) {
-            for (uint32_t li = 0; li < L && rc == ASDM_OK; ++li)
-                if (local_out[live[li]] &&
-                    cudaMemcpyAsync(local_out[live[li]], d_local + local_base[li],
-                                    (local_base[li + 1] - local_base[li]) * sizeof(unsigned long long),
-                                    cudaMemcpyDeviceToHost, s) != cudaSuccess)
-                    rc = fail(ASDM_ERR_CUDA, "local-count readback failed");
-            if (rc == ASDM_OK && cudaStreamSynchronize(s) != cudaSuccess) rc = fail(ASDM_ERR_CUDA, "local-count readback failed");
+            std::vector<LocalRead> reads;
+            for (uint32_t li = 0; li < L; ++li)
+                if (local_out[live[li]]) reads.push_back(LocalRead{cs[live[li]], d_local + local_base[li], local_out[live[li]]});
+            if (!reads.empty()) rc = read_locals(G, reads, *fill);
         }
     } while (false);
     if (e0) cudaEventDestroy(e0);
