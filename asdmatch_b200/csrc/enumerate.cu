@@ -34,7 +34,6 @@
 namespace asdm {
 
 int build_plan(const asdm_cs &cs, const uint32_t *user_order, asdm_plan &p, const asdm_card *card = nullptr);
-bool tree_countable(const QueryGraph &q);
 bool tree_countable_conflicts(const QueryGraph &q);
 int tree_counts(asdm_graph *G, const std::vector<asdm_cs *> &cs, std::vector<uint64_t> &counts,
                 std::vector<char> &done, const std::vector<unsigned long long *> *local = nullptr);
@@ -1873,8 +1872,8 @@ int run_plan(asdm_cs &cs, const asdm_plan &plan, const asdm_run_opts &opt, asdm_
     HostFill fill;
     if (opt.local_counts && (mode & ASDM_MODE_LOCAL)) fill.start({{opt.local_counts, (uint64_t)G->d.n * n}});
     if (!cs.nonempty) return ASDM_OK;
-    if (mode == ASDM_MODE_LOCAL && opt.local_counts && plan.order.size() == n && tree_countable(q)) {
-        // conflict-free tree: counts and local counts from the tree program
+    if (mode == ASDM_MODE_LOCAL && opt.local_counts && plan.order.size() == n && tree_countable_conflicts(q)) {
+        // tree: counts and local counts from the tree program
         const uint64_t local_n = (uint64_t)G->d.n * n;
         unsigned long long *blk = nullptr;
         ASDM_TRY(dalloc(&blk, local_n, s));
@@ -2111,8 +2110,8 @@ int run_plan(asdm_cs &cs, const asdm_plan &plan, const asdm_run_opts &opt, asdm_
 // Batched form: one persistent launch counts every query of a group.
 // counts[i] / status[i] receive each query's result.
 // Queries settled without enumeration, before any plan is needed: tree
-// queries counted by the tree program (in LOCAL mode the conflict-free ones,
-// with their local counts, a few queries at a time), then queries whose count
+// queries counted by the tree program (in LOCAL mode with their local counts,
+// a few queries at a time), then queries whose count
 // a device lower bound shows to be at least 2^64 (ASDM_ERR_OVERFLOW).  Only
 // queries with full[i] set (whole queries, not prefixes) take part.  live
 // holds the positions still open on entry and on return; counts and status of
@@ -2127,7 +2126,7 @@ int settle_queries(asdm_graph *G, const std::vector<asdm_cs *> &cs, const std::v
     if (local_out) {
         std::vector<uint32_t> tid;
         for (uint32_t i : live)
-            if (full[i] && tree_countable(cs[i]->q)) tid.push_back(i);
+            if (full[i] && tree_countable_conflicts(cs[i]->q)) tid.push_back(i);
         std::vector<char> settled(Q, 0);
         cudaEvent_t t0, t1;
         cudaEventCreate(&t0);

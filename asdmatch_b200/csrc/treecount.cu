@@ -65,23 +65,33 @@ struct TreeChild {
     const uint32_t *src;              // map C(r) -> C(u) when u is not the representative (else null)
 };
 
-// Local counts, top down: up_c(j) = sum over i in list_{c->u}(j) of
-// up_u(i) * prod over c's siblings c' of S_{u,c'}(i), with up = 1 at the root.
+// Local counts, top down, for every term: block c hangs on block B by the query
+// edge (member f of B, c's representative);
+//   up_c(j) = sum over i in list_{c->f}(j) of [i is a candidate of every member
+//             of B] * up_B(i) * prod over c's siblings c' of S_{B,c'}(i),
+// with up = 1 at the root and i taken to C(B's representative).
 struct UpSeg {
     unsigned long long *up;             // up_c (output), by candidate of c
-    const uint32_t *off, *list;         // candidate edges (c -> u): for j in C(c), indices into C(u)
-    const unsigned long long *up_u;     // null when u is the root
-    uint32_t sib_first, nsib;           // S arrays of u's other children
+    const uint32_t *off, *list;         // candidate edges (c -> f): for j in C(c), indices into C(f)
+    const uint32_t *src;                // map C(f) -> C(rep of B) when f is not the representative (else null)
+    const unsigned long long *up_u;     // up_B; null when B is the root
+    uint32_t sib_first, nsib;           // S arrays of B's other children
+    uint32_t val_first, nval;           // B's other members' maps
     uint32_t query, ncand;
+    uint32_t check, pad;                // 1: the identity partition's program (overflow checked)
     unsigned long long start;
 };
 
-// local[v][u] = w_u(i) * up_u(i) for v = C(u)[i]
+// local[v][u] += mu(pi) * w_b(i) * up_b(i) for v = C(rep of b)[i] and every
+// member u of block b: the embeddings that send u to v, by the same
+// inclusion-exclusion as their total.
 struct LocSeg {
-    const unsigned long long *w, *up;   // w null at a leaf, up null at the root
+    const unsigned long long *w, *up;   // w null at a one-vertex leaf, up null at the root
     const uint32_t *cand;
     unsigned long long *local;          // |Vg| x n block of the query
+    long long coef;
     uint32_t n, u, query, ncand;
+    uint32_t check, pad;
     unsigned long long start;
 };
 
@@ -228,7 +238,8 @@ __device__ __forceinline__ uint32_t seg_of(const unsigned long long *starts_base
 }
 
 __global__ void tree_up(const UpSeg *__restrict__ segs, uint32_t nseg, unsigned long long total,
-                        const unsigned long long *const *__restrict__ sibs, unsigned int *__restrict__ overflow) {
+                        const unsigned long long *const *__restrict__ sibs, const uint32_t *const *__restrict__ maps,
+                        unsigned int *__restrict__ overflow) {
     for (unsigned long long t = (unsigned long long)blockIdx.x * blockDim.x + threadIdx.x; t < total;
          t += (unsigned long long)gridDim.x * blockDim.x) {
         const UpSeg sg = segs[seg_of(&segs[0].start, sizeof(UpSeg), nseg, t)];
@@ -236,7 +247,11 @@ __global__ void tree_up(const UpSeg *__restrict__ segs, uint32_t nseg, unsigned 
         unsigned long long sum = 0;
         bool over = false;
         for (uint32_t e = sg.off[j]; e < sg.off[j + 1]; ++e) {
-            const uint32_t i = sg.list[e];
+            uint32_t i = sg.list[e];
+            if (sg.src) i = sg.src[i];
+            bool in = i != kNone;
+            for (uint32_t k = 0; k < sg.nval && in; ++k) in = maps[sg.val_first + k][i] != kNone;
+            if (!in) continue;
             unsigned long long x = sg.up_u ? sg.up_u[i] : 1ull;
             for (uint32_t k = 0; k < sg.nsib && x; ++k) {
                 const unsigned long long y = sibs[sg.sib_first + k][i];
@@ -246,7 +261,7 @@ __global__ void tree_up(const UpSeg *__restrict__ segs, uint32_t nseg, unsigned 
             over |= sum + x < sum;
             sum += x;
         }
-        if (over) {
+        if (over && sg.check) {
             atomicOr(&overflow[sg.query], 1u);
             sum = 0;
         }
@@ -261,8 +276,9 @@ __global__ void tree_local(const LocSeg *__restrict__ segs, uint32_t nseg, unsig
         const LocSeg sg = segs[seg_of(&segs[0].start, sizeof(LocSeg), nseg, t)];
         const uint32_t i = (uint32_t)(t - sg.start);
         const unsigned long long a = sg.w ? sg.w[i] : 1ull, b = sg.up ? sg.up[i] : 1ull;
-        if (__umul64hi(a, b) != 0) atomicOr(&overflow[sg.query], 1u);
-        sg.local[(unsigned long long)sg.cand[i] * sg.n + sg.u] = a * b;
+        if (sg.check && __umul64hi(a, b) != 0) atomicOr(&overflow[sg.query], 1u);
+        const unsigned long long x = (unsigned long long)sg.coef * (a * b);
+        if (x) atomicAdd(&sg.local[(unsigned long long)sg.cand[i] * sg.n + sg.u], x);
     }
 }
 
@@ -429,17 +445,7 @@ bool block_trees(const QueryGraph &q, std::vector<BlockTree> &out, const asdm_cs
 
 }  // namespace
 
-// A query whose count (and local counts) the program gives with the identity
-// partition alone: connected tree, no two non-adjacent vertices with one label.
-bool tree_countable(const QueryGraph &q) {
-    if (q.n < 2 || q.off[q.n] != 2 * (q.n - 1)) return false;
-    for (uint32_t u = 0; u < q.n; ++u)
-        for (uint32_t w = u + 1; w < q.n; ++w)
-            if (q.lab[u] == q.lab[w] && q.slot(u, w) < 0) return false;
-    return true;
-}
-
-// A tree query whose count the program gives by inclusion-exclusion: every
+// A tree query whose count (and local counts) the program gives by inclusion-exclusion: every
 // quotient by same-label blocks is a tree (always so when the same-label
 // vertices are at distance 2: siblings, or grandparent and grandchild).
 bool tree_countable_conflicts(const QueryGraph &q) {
@@ -464,14 +470,22 @@ int tree_counts_chunk(asdm_graph *G, const std::vector<asdm_cs *> &cs, std::vect
     std::vector<std::vector<std::vector<uint64_t>>> woff(Q);  // first weight of (query, term, block)
     uint64_t wtotal = 0;
     std::vector<uint32_t> take;
-    // maps C(rep) -> C(member) of merged blocks, one per (query, rep, member)
+    // maps between the candidates of two members of a block, one per (query, from, to)
     std::vector<MapSeg> msegs;
-    std::vector<std::vector<std::pair<uint64_t, uint32_t>>> mkey(Q);  // ((rep << 32) | member, seg)
+    std::vector<std::vector<std::pair<uint64_t, uint32_t>>> mkey(Q);  // ((from << 32) | to, seg)
     uint64_t mtotal = 0;
+    auto add_map = [&](uint32_t qi, uint32_t from, uint32_t to) {
+        const asdm_cs &c = *cs[qi];
+        const uint64_t key = ((uint64_t)from << 32) | to;
+        for (auto &kv : mkey[qi])
+            if (kv.first == key) return;
+        mkey[qi].emplace_back(key, (uint32_t)msegs.size());
+        msegs.push_back(MapSeg{c.d_cand + c.cand_base[from], c.d_cand + c.cand_base[to], nullptr, c.ncand[to], 0, mtotal});
+        mtotal += c.ncand[from];
+    };
     for (uint32_t qi = 0; qi < Q; ++qi) {
         const asdm_cs &c = *cs[qi];
         if (!c.nonempty || !block_trees(c.q, trees[qi], &c)) continue;
-        if (local && trees[qi].size() != 1) continue;
         woff[qi].resize(trees[qi].size());
         for (uint32_t ti = 0; ti < trees[qi].size(); ++ti) {
             const BlockTree &t = trees[qi][ti];
@@ -483,17 +497,11 @@ int tree_counts_chunk(asdm_graph *G, const std::vector<asdm_cs *> &cs, std::vect
                 by_height[t.height[b]].push_back(Item{qi, ti, b});
                 if (by_depth.size() <= t.depth[b]) by_depth.resize(t.depth[b] + 1);
                 by_depth[t.depth[b]].push_back(Item{qi, ti, b});
-                for (uint32_t u : t.members[b]) {
-                    if (u == t.rep[b]) continue;
-                    const uint64_t key = ((uint64_t)t.rep[b] << 32) | u;
-                    bool have = false;
-                    for (auto &kv : mkey[qi]) have = have || kv.first == key;
-                    if (have) continue;
-                    mkey[qi].emplace_back(key, (uint32_t)msegs.size());
-                    msegs.push_back(MapSeg{c.d_cand + c.cand_base[t.rep[b]], c.d_cand + c.cand_base[u], nullptr,
-                                           c.ncand[u], 0, mtotal});
-                    mtotal += c.ncand[t.rep[b]];
-                }
+                for (uint32_t u : t.members[b])
+                    if (u != t.rep[b]) add_map(qi, t.rep[b], u);
+                // the way up from a child of a member that is not the representative
+                if (local && t.parent[b] != kNone && t.pfrom[b] != t.rep[t.parent[b]])
+                    add_map(qi, t.pfrom[b], t.rep[t.parent[b]]);
             }
         }
         take.push_back(qi);
@@ -503,30 +511,32 @@ int tree_counts_chunk(asdm_graph *G, const std::vector<asdm_cs *> &cs, std::vect
         const BlockTree &t = trees[qi][ti];
         return t.height[b] == 0 && t.members[b].size() == 1;
     };
-    auto wptr_off = [&](uint32_t qi, uint32_t u) { return woff[qi][0][u]; };  // identity term: block = vertex
-    // S_{parent(c), c} has |C(parent)| entries, at sslot[query][c]
-    std::vector<std::vector<uint64_t>> sslot(Q);
+    // local counts: S_{B, c} has |C(rep of B)| entries, at sslot[query][term][c]
+    std::vector<std::vector<std::vector<uint64_t>>> sslot(Q);
     uint64_t stotal = 0;
     if (local) {
-        for (uint32_t qi : take) sslot[qi].assign(cs[qi]->q.n, 0);
-        for (const auto &lv : by_height)
-            for (const Item &it : lv) {
-                const uint32_t par = trees[it.q][it.t].parent[it.b];
-                if (par != kNone) {
-                    sslot[it.q][it.b] = stotal;
-                    stotal += cs[it.q]->ncand[par];
-                }
+        for (uint32_t qi : take) {
+            sslot[qi].resize(trees[qi].size());
+            for (size_t ti = 0; ti < trees[qi].size(); ++ti) {
+                const BlockTree &t = trees[qi][ti];
+                sslot[qi][ti].assign(t.nb, 0);
+                for (uint32_t b = 0; b < t.nb; ++b)
+                    if (t.parent[b] != kNone) {
+                        sslot[qi][ti][b] = stotal;
+                        stotal += cs[qi]->ncand[t.rep[t.parent[b]]];
+                    }
             }
+        }
     }
     unsigned long long *sbase = nullptr;
-    auto s_of = [&](uint32_t qi, uint32_t ch) { return sbase + sslot[qi][ch]; };
+    auto s_of = [&](uint32_t qi, uint32_t ti, uint32_t ch) { return sbase + sslot[qi][ti][ch]; };
     unsigned long long *w = nullptr, *d_counts = nullptr, *d_homs = nullptr, *sums = nullptr, *up = nullptr;
     unsigned int *d_over = nullptr;
     uint32_t *d_mapbuf = nullptr;
     TreeSeg *d_segs = nullptr;
     TreeChild *d_kids = nullptr;
     MapSeg *d_mseg = nullptr;
-    const uint32_t **d_maps = nullptr;
+    const uint32_t **d_maps = nullptr, **d_upmaps = nullptr;
     UpSeg *d_up = nullptr;
     LocSeg *d_loc = nullptr;
     const unsigned long long **d_sibs = nullptr;
@@ -600,7 +610,7 @@ int tree_counts_chunk(asdm_graph *G, const std::vector<asdm_cs *> &cs, std::vect
                     const uint32_t e = t.pedge[C], u = t.pfrom[C];
                     kids.push_back(TreeChild{c.d_eoff + c.eoff_base[e], c.d_elist + c.elist_base[e],
                                              is_leaf1(it.q, it.t, C) ? nullptr : w + woff[it.q][it.t][C],
-                                             local ? s_of(it.q, C) : nullptr, u == r ? nullptr : map_of(it.q, r, u)});
+                                             local ? s_of(it.q, it.t, C) : nullptr, u == r ? nullptr : map_of(it.q, r, u)});
                 }
                 (void)q;
                 sg.nchild = (uint32_t)kids.size() - sg.child_first;
@@ -638,6 +648,7 @@ int tree_counts_chunk(asdm_graph *G, const std::vector<asdm_cs *> &cs, std::vect
         if (rc != ASDM_OK) break;
         std::vector<UpSeg> ups;
         std::vector<const unsigned long long *> sibs;
+        std::vector<const uint32_t *> upmaps;
         std::vector<size_t> dfirst{0};
         std::vector<unsigned long long> dtotal;
         std::vector<LocSeg> locs;
@@ -647,26 +658,28 @@ int tree_counts_chunk(asdm_graph *G, const std::vector<asdm_cs *> &cs, std::vect
             for (size_t dpt = 1; dpt < by_depth.size(); ++dpt) {
                 unsigned long long total = 0;
                 for (const Item &it : by_depth[dpt]) {
-                    // identity terms only: block b is vertex b
                     const asdm_cs &c = *cs[it.q];
                     const QueryGraph &q = c.q;
-                    const std::vector<uint32_t> &par = trees[it.q][0].parent;
-                    const uint32_t u = par[it.b];
-                    const int k = q.slot(it.b, u);  // edge (c -> u)
-                    const uint32_t e = q.off[it.b] + (uint32_t)k;
+                    const BlockTree &t = trees[it.q][it.t];
+                    const uint32_t B = t.parent[it.b], r = t.rep[it.b], f = t.pfrom[it.b], rB = t.rep[B];
+                    const uint32_t e = q.off[r] + (uint32_t)q.slot(r, f);  // edge (r -> f)
                     UpSeg sg{};
-                    sg.up = up + wptr_off(it.q, it.b);
+                    sg.up = up + woff[it.q][it.t][it.b];
                     sg.off = c.d_eoff + c.eoff_base[e];
                     sg.list = c.d_elist + c.elist_base[e];
-                    sg.up_u = par[u] == kNone ? nullptr : up + wptr_off(it.q, u);
+                    sg.src = f == rB ? nullptr : map_of(it.q, f, rB);
+                    sg.up_u = t.parent[B] == kNone ? nullptr : up + woff[it.q][it.t][B];
                     sg.sib_first = (uint32_t)sibs.size();
-                    for (uint32_t e2 = q.off[u]; e2 < q.off[u + 1]; ++e2) {
-                        const uint32_t c2 = q.nbr[e2];
-                        if (par[c2] == u && c2 != it.b) sibs.push_back(s_of(it.q, c2));
-                    }
+                    for (uint32_t C = 0; C < t.nb; ++C)
+                        if (t.parent[C] == B && C != it.b) sibs.push_back(s_of(it.q, it.t, C));
                     sg.nsib = (uint32_t)sibs.size() - sg.sib_first;
+                    sg.val_first = (uint32_t)upmaps.size();
+                    for (uint32_t u : t.members[B])
+                        if (u != rB) upmaps.push_back(map_of(it.q, rB, u));
+                    sg.nval = (uint32_t)upmaps.size() - sg.val_first;
                     sg.query = it.q;
-                    sg.ncand = c.ncand[it.b];
+                    sg.ncand = c.ncand[r];
+                    sg.check = t.identity ? 1u : 0u;
                     sg.start = total;
                     total += sg.ncand;
                     ups.push_back(sg);
@@ -676,24 +689,32 @@ int tree_counts_chunk(asdm_graph *G, const std::vector<asdm_cs *> &cs, std::vect
             }
             for (uint32_t qi : take) {
                 const asdm_cs &c = *cs[qi];
-                for (uint32_t u = 0; u < c.q.n; ++u) {
-                    const bool root = trees[qi][0].parent[u] == kNone;
-                    LocSeg ls{is_leaf1(qi, 0, u) ? nullptr : w + wptr_off(qi, u), root ? nullptr : up + wptr_off(qi, u),
-                              c.d_cand + c.cand_base[u], (*local)[qi], c.q.n, u, qi, c.ncand[u], ltotal};
-                    ltotal += c.ncand[u];
-                    locs.push_back(ls);
+                for (uint32_t ti = 0; ti < trees[qi].size(); ++ti) {
+                    const BlockTree &t = trees[qi][ti];
+                    for (uint32_t b = 0; b < t.nb; ++b)
+                        for (uint32_t u : t.members[b]) {
+                            LocSeg ls{is_leaf1(qi, ti, b) ? nullptr : w + woff[qi][ti][b],
+                                      t.parent[b] == kNone ? nullptr : up + woff[qi][ti][b],
+                                      c.d_cand + c.cand_base[t.rep[b]], (*local)[qi], t.coef, c.q.n, u, qi,
+                                      c.ncand[t.rep[b]], t.identity ? 1u : 0u, 0, ltotal};
+                            ltotal += c.ncand[t.rep[b]];
+                            locs.push_back(ls);
+                        }
                 }
             }
+            if (upmaps.empty()) upmaps.push_back(nullptr);
             if (sibs.empty()) sibs.push_back(nullptr);
             if (ups.empty()) ups.push_back(UpSeg{});
             if ((rc = dalloc(&d_up, ups.size(), s)) || (rc = dalloc(&d_sibs, sibs.size(), s)) ||
-                (rc = dalloc(&d_loc, locs.size(), s)))
+                (rc = dalloc(&d_loc, locs.size(), s)) || (rc = dalloc(&d_upmaps, upmaps.size(), s)))
                 break;
             if (cudaMemcpyAsync(d_up, ups.data(), ups.size() * sizeof(UpSeg), cudaMemcpyHostToDevice, s) !=
                     cudaSuccess ||
                 cudaMemcpyAsync(d_sibs, sibs.data(), sibs.size() * sizeof(void *), cudaMemcpyHostToDevice, s) !=
                     cudaSuccess ||
                 cudaMemcpyAsync(d_loc, locs.data(), locs.size() * sizeof(LocSeg), cudaMemcpyHostToDevice, s) !=
+                    cudaSuccess ||
+                cudaMemcpyAsync(d_upmaps, upmaps.data(), upmaps.size() * sizeof(void *), cudaMemcpyHostToDevice, s) !=
                     cudaSuccess) {
                 rc = fail(ASDM_ERR_CUDA, "tree local-count upload failed");
                 break;
@@ -703,7 +724,7 @@ int tree_counts_chunk(asdm_graph *G, const std::vector<asdm_cs *> &cs, std::vect
                 const unsigned grid = (unsigned)std::min<unsigned long long>((dtotal[k] + 255) / 256,
                                                                              (unsigned long long)G->num_sms * 32);
                 tree_up<<<grid, 256, 0, s>>>(d_up + dfirst[k], (uint32_t)(dfirst[k + 1] - dfirst[k]), dtotal[k], d_sibs,
-                                             d_over);
+                                             d_upmaps, d_over);
                 ::asdm::count_launch();
                 if (cudaGetLastError() != cudaSuccess) rc = fail(ASDM_ERR_CUDA, "tree local-count kernel failed");
             }
@@ -739,6 +760,7 @@ int tree_counts_chunk(asdm_graph *G, const std::vector<asdm_cs *> &cs, std::vect
     dfree(d_up, s);
     dfree(d_sibs, s);
     dfree(d_loc, s);
+    dfree(d_upmaps, s);
     dfree(sums, s);
     dfree(up, s);
     dfree(w, s);
@@ -2489,7 +2511,7 @@ int overflow_bounds(asdm_graph *G, const std::vector<asdm_cs *> &cs, std::vector
 
 // Counts every countable query of `cs` (non-empty candidate spaces on graph
 // G); done[i] = 1 and counts[i] set for the queries it settled.  With local
-// counts only queries without conflicts are taken.  Queries run in chunks of
+// counts the top-down pass of every term follows.  Queries run in chunks of
 // at most kTreeChunkWords device words (one query alone may exceed it).
 int tree_counts(asdm_graph *G, const std::vector<asdm_cs *> &cs, std::vector<uint64_t> &counts,
                 std::vector<char> &done, const std::vector<unsigned long long *> *local) {
@@ -2503,7 +2525,7 @@ int tree_counts(asdm_graph *G, const std::vector<asdm_cs *> &cs, std::vector<uin
         std::vector<size_t> ids;
         uint64_t words = 0;
         for (; at < Q; ++at) {
-            const uint64_t w = tree_words(*cs[at]);
+            const uint64_t w = tree_words(*cs[at]) * (local ? 3 : 1);  // list sums and the way up beside the weights
             if (!ids.empty() && words + w > kTreeChunkWords) break;
             words += w;
             part.push_back(cs[at]);
