@@ -862,7 +862,10 @@ struct Warp {
 
     // Loads the candidate-edge lists of level d's earlier neighbours into the
     // level's slots and picks the shortest as driver.  Returns its length.
-    __device__ uint32_t setup(uint32_t d, bool whole = true) {
+    // When level d - 1 was just given candidate x, vx is its vertex, loaded by
+    // lane 0 and stored here: its load and the lists' offsets are in flight
+    // together (one latency per node instead of two).
+    __device__ uint32_t setup(uint32_t d, bool whole, bool opened, uint32_t vx) {
         const DLevel lv = L[d];
         uint32_t s_len = 0xFFFFFFFFu;
         if (lane < lv.nback) {
@@ -874,15 +877,10 @@ struct Warp {
             slen[lv.back_first + lane] = s_len;
             scur[lv.back_first + lane] = 0;
         }
-        uint32_t key = s_len, who = lane;
-#pragma unroll
-        for (int o = 16; o; o >>= 1) {
-            const uint32_t k2 = __shfl_xor_sync(kFull, key, o), w2 = __shfl_xor_sync(kFull, who, o);
-            if (k2 < key || (k2 == key && w2 < who)) { key = k2; who = w2; }
-        }
-        uint32_t tot = lane < lv.nback ? s_len : 0;
-#pragma unroll
-        for (int o = 16; o; o >>= 1) tot += __shfl_xor_sync(kFull, tot, o);
+        if (opened && lane == 0) vid[d - 1] = vx;
+        const uint32_t key = __reduce_min_sync(kFull, s_len);
+        const uint32_t who = __ffs(__ballot_sync(kFull, lane < lv.nback && s_len == key)) - 1;  // the first shortest
+        const uint32_t tot = __reduce_add_sync(kFull, lane < lv.nback ? s_len : 0u);
         // a counted last level with one list reads only its two offsets; a
         // level searched over part of its driver list is counted by the caller
         if (whole) elems += (MODE == ASDM_MODE_COUNT && d + 1 == n && lv.nback == 1) ? 2 : tot;
@@ -1318,15 +1316,16 @@ __device__ bool dfs(const EnumArgs &a, Warp<MODE, MULTI> &W, uint32_t lane, uint
         if (W.pos[d] < W.cnt[d]) {
             const uint32_t x = W.buf[32 * d + W.pos[d]];
             __syncwarp();
+            uint32_t vx = 0;
             if (lane == 0) {
+                vx = W.L[d].cand[x];
                 W.pos[d] += 1;
                 W.idx[d] = x;
-                W.vid[d] = W.L[d].cand[x];
             }
             __syncwarp();
             ++d;
             const bool closed = W.closed_at(d);
-            const uint32_t len = W.setup(d, !closed);
+            const uint32_t len = W.setup(d, !closed, true, vx);
             if (closed) {
                 if (len) {
                     W.prepare_lane_leaf(d);
@@ -1360,14 +1359,14 @@ template <uint32_t MODE, bool MULTI>
 __device__ __forceinline__ bool run_range(const EnumArgs &a, Warp<MODE, MULTI> &W, uint32_t lane, uint32_t s, uint32_t lo, uint32_t hi,
                           uint32_t &iter, uint64_t deadline) {
     if (W.closed_at(s)) {
-        W.setup(s, false);
+        W.setup(s, false, false, 0);
         if (hi > lo) {
             W.prepare_lane_leaf(s);
             W.tail2(s, lo, hi);
         }
         return true;
     }
-    W.setup(s, false);
+    W.setup(s, false, false, 0);
     {
         // list entries this range touches: the driver positions [lo, hi), one
         // probe of every other list per driver entry, and the lists' offsets
