@@ -763,6 +763,9 @@ unsigned grid_for(uint64_t items, int num_sms) {
 // Candidate arrays of at most this many entries in total are allocated for
 // their bound, |V_l(u)| each, so the host need not read their sizes first.
 constexpr uint64_t kCandBound = 1u << 20;
+// Items and possible list entries of a group small enough for K3's short form,
+// and the possible entries whose memory (4 MiB) is not worth a readback.
+constexpr uint64_t kSmallItems = 1u << 16, kSmallLists = 1u << 22, kListBound = 1u << 20;
 
 struct Scratch {
     cudaStream_t s;
@@ -1156,6 +1159,7 @@ int build_batch(const std::vector<asdm_cs *> &group) {
     std::vector<EdgeDesc> edges;
     std::vector<uint64_t> item_base{0};
     std::vector<uint32_t> edge_first(Q, 0);
+    uint64_t list_bound = 0;  // of all lists: at most |C(u2)| or the largest degree each
     for (uint32_t qi = 0; qi < Q; ++qi) {
         const QPlan &qp = P[qi];
         edge_first[qi] = (uint32_t)edges.size();
@@ -1169,6 +1173,7 @@ int build_batch(const std::vector<asdm_cs *> &group) {
                 edges.push_back(
                     EdgeDesc{arena->d_cand + cs.cand_base[u], (uint32_t)mword[s2], cs.ncand[u], q.lab[u2], 0});
                 item_base.push_back(item_base.back() + cs.ncand[u] + 1);
+                list_bound += (uint64_t)cs.ncand[u] * std::min(cs.ncand[u2], G->max_deg);
             }
     }
     const uint32_t ne = (uint32_t)edges.size();
@@ -1196,70 +1201,94 @@ int build_batch(const std::vector<asdm_cs *> &group) {
         uint64_t bound = 0;
         uint32_t *rstart = nullptr;
         uint64_t *d_upos = nullptr;
-        ASDM_TRY(scr.alloc(&rstart, nitems));
-        ASDM_TRY(scr.alloc(&d_upos, nitems + 1));
-        k3_bound<<<egrid, kBlock, 0, s>>>(g, d_edges, d_ib, ne, arena->d_eoff, rstart);
-        ::asdm::count_launch();
-        ASDM_CUDA(cudaGetLastError());
-        ASDM_TRY(scan_exclusive_u32(arena->d_eoff, d_upos, nitems, true, s));
-        ASDM_CUDA(cudaMemcpyAsync(&bound, d_upos + nitems, sizeof(uint64_t), cudaMemcpyDeviceToHost, s));
-        ASDM_CUDA(cudaStreamSynchronize(s));
-        // staging buffers of up to 2^padded_cap_log2 entries (default 2^33: 32 GiB)
+        // Small groups take the two-scan form too, whose four launches and no
+        // size readback are quicker than the chunked fill's eight and two
+        // (one 8-vertex query on 3,112 vertices: 490 -> 404 us a call).  Up to
+        // kListBound possible entries the lists get room for all of them; beyond,
+        // their exact length is read back first.  A group whose lists could pass
+        // the staging cap is not small: the cap decides about it below.
         const uint64_t padded_cap = 1ull << G->tuning.padded_cap_log2;
-        two_scan = bound > padded_cap || nitems >= 0xFFFFFF00ull;  // k3_fill numbers items in 32 bits
-        if (!two_scan) {
-            const uint32_t clog = chunk_log2_for(bound, G->num_sms);
-            const uint32_t nchunks = (uint32_t)std::max<uint64_t>(1, (bound + (1ull << clog) - 1) >> clog);
-            uint2 *d_chunk = nullptr;  // the chunks' first items
-            uint32_t *d_stage = nullptr, *d_chits = nullptr;
-            uint64_t *d_cbase = nullptr;
-            ASDM_TRY(scr.alloc(&d_stage, (uint64_t)nchunks << clog));
-            ASDM_TRY(scr.alloc(&d_chunk, nchunks));
-            ASDM_TRY(scr.alloc(&d_chits, nchunks));
-            ASDM_TRY(scr.alloc(&d_cbase, (uint64_t)nchunks + 1));
-            if (bound == 0) ASDM_CUDA(cudaMemsetAsync(d_chunk, 0, sizeof(uint2), s));
-            k3_chunks<<<egrid, kBlock, 0, s>>>(d_ib, ne, d_upos, clog, d_chunk);
-            ::asdm::count_launch();
-            const unsigned cgrid = grid_for(32ull * nchunks, G->num_sms);  // a warp per chunk
-            k3_fill<<<cgrid, kBlock, 0, s>>>(g, d_edges, cmem, d_ib, ne, d_upos, rstart, d_chunk, nchunks, clog,
-                                             arena->d_eoff, d_stage, d_chits);
-            ::asdm::count_launch();
-            ASDM_CUDA(cudaGetLastError());
-            ASDM_TRY(scan_exclusive_u32(d_chits, d_cbase, nchunks, true, s));
-            ASDM_CUDA(cudaMemcpyAsync(&total, d_cbase + nchunks, sizeof(uint64_t), cudaMemcpyDeviceToHost, s));
-            k3_starts<<<(ne + kBlock - 1) / kBlock, kBlock, 0, s>>>(d_ib, ne, d_upos, nchunks, clog, d_cbase, arena->d_eoff,
-                                                                   d_estart);
-            ::asdm::count_launch();
-            k3_rebase<<<egrid, kBlock, 0, s>>>(d_ib, ne, d_upos, nchunks, clog, d_cbase, d_estart, arena->d_eoff);
-            ::asdm::count_launch();
-            ASDM_CUDA(cudaStreamSynchronize(s));
-            ASDM_TRY(dalloc(&arena->d_elist, total, s));
-            k3_pack<<<cgrid, kBlock, 0, s>>>(d_stage, d_chits, d_cbase, nchunks, clog, arena->d_elist);
-            ::asdm::count_launch();
-            ASDM_CUDA(cudaGetLastError());
-            run_entries = bound;
-        } else {
+        const bool small = nitems <= kSmallItems && list_bound <= std::min(kSmallLists, padded_cap);
+        if (small) {
             ASDM_TRY(scr.alloc(&d_wpos, nitems + 1));
             k3_edges<false><<<egrid, kBlock, 0, s>>>(g, d_edges, cmem, d_ib, ne, arena->d_eoff, nullptr, nullptr,
                                                     d_elems + 1, nullptr);
             ::asdm::count_launch();
-            ASDM_CUDA(cudaGetLastError());
             ASDM_TRY(scan_exclusive_u32(arena->d_eoff, d_wpos, nitems, true, s));
             ASDM_CUDA(cudaMemcpyAsync(&total, d_wpos + nitems, sizeof(uint64_t), cudaMemcpyDeviceToHost, s));
-            ASDM_CUDA(cudaStreamSynchronize(s));
-            ASDM_TRY(dalloc(&arena->d_elist, total, s));
+            if (list_bound > kListBound) ASDM_CUDA(cudaStreamSynchronize(s));
+            ASDM_TRY(dalloc(&arena->d_elist, list_bound > kListBound ? total : list_bound, s));
             k3_edges<true><<<egrid, kBlock, 0, s>>>(g, d_edges, cmem, d_ib, ne, nullptr, d_wpos, arena->d_elist,
                                                     nullptr, nullptr);
             ::asdm::count_launch();
-            ASDM_CUDA(cudaGetLastError());
-            k3_offsets<<<grid_for(nitems, G->num_sms), kBlock, 0, s>>>(d_ib, ne, d_wpos, arena->d_eoff, d_estart,
-                                                                      d_bad);
+            k3_offsets<<<egrid, kBlock, 0, s>>>(d_ib, ne, d_wpos, arena->d_eoff, d_estart, d_bad);
             ::asdm::count_launch();
             ASDM_CUDA(cudaGetLastError());
+        } else {
+            ASDM_TRY(scr.alloc(&rstart, nitems));
+            ASDM_TRY(scr.alloc(&d_upos, nitems + 1));
+            k3_bound<<<egrid, kBlock, 0, s>>>(g, d_edges, d_ib, ne, arena->d_eoff, rstart);
+            ::asdm::count_launch();
+            ASDM_CUDA(cudaGetLastError());
+            ASDM_TRY(scan_exclusive_u32(arena->d_eoff, d_upos, nitems, true, s));
+            ASDM_CUDA(cudaMemcpyAsync(&bound, d_upos + nitems, sizeof(uint64_t), cudaMemcpyDeviceToHost, s));
+            ASDM_CUDA(cudaStreamSynchronize(s));
+            // staging buffers of up to 2^padded_cap_log2 entries (default 2^33: 32 GiB)
+            two_scan = bound > padded_cap || nitems >= 0xFFFFFF00ull;  // k3_fill numbers items in 32 bits
+            if (!two_scan) {
+                const uint32_t clog = chunk_log2_for(bound, G->num_sms);
+                const uint32_t nchunks = (uint32_t)std::max<uint64_t>(1, (bound + (1ull << clog) - 1) >> clog);
+                uint2 *d_chunk = nullptr;  // the chunks' first items
+                uint32_t *d_stage = nullptr, *d_chits = nullptr;
+                uint64_t *d_cbase = nullptr;
+                ASDM_TRY(scr.alloc(&d_stage, (uint64_t)nchunks << clog));
+                ASDM_TRY(scr.alloc(&d_chunk, nchunks));
+                ASDM_TRY(scr.alloc(&d_chits, nchunks));
+                ASDM_TRY(scr.alloc(&d_cbase, (uint64_t)nchunks + 1));
+                if (bound == 0) ASDM_CUDA(cudaMemsetAsync(d_chunk, 0, sizeof(uint2), s));
+                k3_chunks<<<egrid, kBlock, 0, s>>>(d_ib, ne, d_upos, clog, d_chunk);
+                ::asdm::count_launch();
+                const unsigned cgrid = grid_for(32ull * nchunks, G->num_sms);  // a warp per chunk
+                k3_fill<<<cgrid, kBlock, 0, s>>>(g, d_edges, cmem, d_ib, ne, d_upos, rstart, d_chunk, nchunks, clog,
+                                                 arena->d_eoff, d_stage, d_chits);
+                ::asdm::count_launch();
+                ASDM_CUDA(cudaGetLastError());
+                ASDM_TRY(scan_exclusive_u32(d_chits, d_cbase, nchunks, true, s));
+                ASDM_CUDA(cudaMemcpyAsync(&total, d_cbase + nchunks, sizeof(uint64_t), cudaMemcpyDeviceToHost, s));
+                k3_starts<<<(ne + kBlock - 1) / kBlock, kBlock, 0, s>>>(d_ib, ne, d_upos, nchunks, clog, d_cbase, arena->d_eoff,
+                                                                       d_estart);
+                ::asdm::count_launch();
+                k3_rebase<<<egrid, kBlock, 0, s>>>(d_ib, ne, d_upos, nchunks, clog, d_cbase, d_estart, arena->d_eoff);
+                ::asdm::count_launch();
+                ASDM_CUDA(cudaStreamSynchronize(s));
+                ASDM_TRY(dalloc(&arena->d_elist, total, s));
+                k3_pack<<<cgrid, kBlock, 0, s>>>(d_stage, d_chits, d_cbase, nchunks, clog, arena->d_elist);
+                ::asdm::count_launch();
+                ASDM_CUDA(cudaGetLastError());
+                run_entries = bound;
+            } else {
+                ASDM_TRY(scr.alloc(&d_wpos, nitems + 1));
+                k3_edges<false><<<egrid, kBlock, 0, s>>>(g, d_edges, cmem, d_ib, ne, arena->d_eoff, nullptr, nullptr,
+                                                        d_elems + 1, nullptr);
+                ::asdm::count_launch();
+                ASDM_CUDA(cudaGetLastError());
+                ASDM_TRY(scan_exclusive_u32(arena->d_eoff, d_wpos, nitems, true, s));
+                ASDM_CUDA(cudaMemcpyAsync(&total, d_wpos + nitems, sizeof(uint64_t), cudaMemcpyDeviceToHost, s));
+                ASDM_CUDA(cudaStreamSynchronize(s));
+                ASDM_TRY(dalloc(&arena->d_elist, total, s));
+                k3_edges<true><<<egrid, kBlock, 0, s>>>(g, d_edges, cmem, d_ib, ne, nullptr, d_wpos, arena->d_elist,
+                                                        nullptr, nullptr);
+                ::asdm::count_launch();
+                ASDM_CUDA(cudaGetLastError());
+                k3_offsets<<<grid_for(nitems, G->num_sms), kBlock, 0, s>>>(d_ib, ne, d_wpos, arena->d_eoff, d_estart,
+                                                                          d_bad);
+                ::asdm::count_launch();
+                ASDM_CUDA(cudaGetLastError());
+            }
         }
         uint32_t bad = 0;
         ASDM_CUDA(cudaMemcpyAsync(estart.data(), d_estart, ne * sizeof(uint64_t), cudaMemcpyDeviceToHost, s));
-        if (two_scan) ASDM_CUDA(cudaMemcpyAsync(&bad, d_bad, sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
+        if (two_scan || small) ASDM_CUDA(cudaMemcpyAsync(&bad, d_bad, sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
         ASDM_CUDA(cudaStreamSynchronize(s));
         for (uint32_t e = 0; e < ne && !bad; ++e)
             bad = (e + 1 < ne ? estart[e + 1] : total) - estart[e] > 0xFFFFFFFFull;

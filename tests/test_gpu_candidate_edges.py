@@ -60,3 +60,11 @@ def test_lists_of_a_biclique(hubs, leaves):
     assert np.array_equal(ids, np.tile(np.arange(hubs), leaves))
     cs.close()
     dg.close()
+
+
+# around the 2^20 possible entries beyond which the short form reads its length back, and the 2^16 items
+# (both directions' candidates and an end each) and 2^22 possible entries beyond which the chunked form runs
+@pytest.mark.parametrize("hubs,leaves", [(512, 1023), (512, 1024), (512, 1025), (2, 65_531), (2, 65_532), (2, 65_533),
+                                         (1447, 1449), (1448, 1449)])
+def test_short_form_limits(hubs, leaves):
+    test_lists_of_a_biclique(hubs, leaves)
