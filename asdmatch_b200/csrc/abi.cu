@@ -348,15 +348,16 @@ extern "C" int asdm_intersect_batch(const uint32_t *values, const uint64_t *list
 }
 
 namespace asdm {
+struct LocalSub;
 int build_plan(const asdm_cs &cs, const uint32_t *user_order, asdm_plan &p, const asdm_card *card = nullptr);
 int build_prefix_plan(const asdm_cs &cs, const uint32_t *order, uint32_t depth, asdm_plan &p);
 int run_batch_count(asdm_graph *G, const std::vector<asdm_cs *> &cs, const std::vector<const asdm_plan *> &plans,
                     double time_limit_s, uint64_t count_limit, uint64_t *counts, int *status, asdm_run_stats *agg,
                     uint64_t *const *local_out, uint64_t *cycles = nullptr, double query_time_s = 0.0,
-                    bool settled = false, HostFill *fill = nullptr);
+                    bool settled = false, HostFill *fill = nullptr, const std::vector<LocalSub> *subs = nullptr);
 int settle_queries(asdm_graph *G, const std::vector<asdm_cs *> &cs, const std::vector<char> &full,
                    std::vector<uint32_t> &live, uint64_t count_limit, uint64_t *counts, int *status,
-                   asdm_run_stats *agg, uint64_t *const *local_out, HostFill *fill = nullptr);
+                   asdm_run_stats *agg, uint64_t *const *local_out, HostFill *fill, bool limited);
 int plan_batch_learned(const std::vector<asdm_cs *> &css, asdm_estimator *e, uint32_t kmax,
                        std::vector<asdm_plan> &plans);
 }  // namespace asdm
@@ -442,7 +443,8 @@ static int run_batch_impl(asdm_graph *g, uint32_t nq, const uint32_t *q_sizes, c
                 for (uint32_t id : ids) slo.push_back(local_out[id]);
             const std::vector<uint32_t> before = live;
             rc = settle_queries(g, group, full, live, count_limit, sc.data(), sst.data(), &gs,
-                                local_out ? slo.data() : nullptr, &fill);
+                                local_out ? slo.data() : nullptr, &fill,
+                                time_limit_s > 0 || query_time_s > 0 || count_limit);
             if (rc != ASDM_OK) {
                 for (uint32_t id : ids) status[id] = rc;
                 if (worst == ASDM_OK) worst = rc;

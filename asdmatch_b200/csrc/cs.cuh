@@ -50,6 +50,27 @@ namespace asdm {
 int build_batch(const std::vector<asdm_cs *> &group);
 }  // namespace asdm
 
+namespace asdm {
+// A tree query with some same-label vertices three or more edges apart merged.
+struct Quotient {
+    QueryGraph q;
+    std::vector<uint32_t> block;  // query vertex -> quotient vertex
+};
+// Fewest maps (see far_quotients) of a query counted through its quotients;
+// with fewer, building their candidate spaces costs more than it saves (one
+// query's local counts on 10^6 vertices, enumerated and through quotients:
+// 3.2 and 3.5 ms at 2^24 maps, 4.9 and 4.9 at 2^29, 8.5 and 6.6 at 2^31, 113
+// and 19 at 2^37).
+constexpr uint64_t kQuotientMaps = 1u << 29;
+// The same by an estimate from averages, asked before the maps are counted.
+// Uneven degrees put it below the count: 2^20.9 to 2^23.8 in the cases above
+// at 2^29 and 2^30 maps, 2^24.2 where quotients first are the faster.  Queries
+// of 4 to 7 vertices on 3,112 vertices stay below 2^19 (one that counts its
+// maps in vain takes 450 us instead of 270).
+constexpr uint64_t kQuotientEstimate = 1u << 24;
+bool far_quotients(const asdm_cs &cs, std::vector<Quotient> &out);
+}  // namespace asdm
+
 struct asdm_plan {
     std::vector<uint32_t> order;                                   // level -> query vertex
     std::vector<std::vector<std::pair<uint32_t, uint32_t>>> back;  // level -> (earlier level j, edge u_j -> u_k)

@@ -1203,7 +1203,7 @@ int build_batch(const std::vector<asdm_cs *> &group) {
         uint64_t *d_upos = nullptr;
         // Small groups take the two-scan form too, whose four launches and no
         // size readback are quicker than the chunked fill's eight and two
-        // (one 8-vertex query on 3,112 vertices: 490 -> 404 us a call).  Up to
+        // (one 8-vertex query on 3,112 vertices: 490 -> 418 us a call).  Up to
         // kListBound possible entries the lists get room for all of them; beyond,
         // their exact length is read back first.  A group whose lists could pass
         // the staging cap is not small: the cap decides about it below.

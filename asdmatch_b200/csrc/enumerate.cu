@@ -36,9 +36,22 @@ namespace asdm {
 int build_plan(const asdm_cs &cs, const uint32_t *user_order, asdm_plan &p, const asdm_card *card = nullptr);
 bool tree_countable_conflicts(const QueryGraph &q);
 int tree_counts(asdm_graph *G, const std::vector<asdm_cs *> &cs, std::vector<uint64_t> &counts,
-                std::vector<char> &done, const std::vector<unsigned long long *> *local = nullptr);
+                std::vector<char> &done, const std::vector<unsigned long long *> *local = nullptr,
+                bool near_only = false);
 int overflow_bounds(asdm_graph *G, const std::vector<asdm_cs *> &cs, std::vector<char> &proven,
                     std::vector<uint64_t> *lower = nullptr);
+
+// A run's local counts are taken off those of a query it is a quotient of:
+// dst[v][u] -= src[v][block[u]] (|Vg| x n and |Vg| x src_n).
+struct LocalSub {
+    unsigned long long *dst = nullptr;
+    uint32_t n = 0, src_n = 0;
+    uint8_t block[kMaxQuery] = {};
+};
+int run_batch_count(asdm_graph *G, const std::vector<asdm_cs *> &cs, const std::vector<const asdm_plan *> &plans,
+                    double time_limit_s, uint64_t count_limit, uint64_t *counts, int *status, asdm_run_stats *agg,
+                    uint64_t *const *local_out, uint64_t *cycles, double query_time_s, bool settled, HostFill *fill,
+                    const std::vector<LocalSub> *subs);
 
 namespace {
 
@@ -1861,6 +1874,92 @@ void root_blocks(const asdm_cs &cs, const asdm_plan &plan, unsigned long long &p
     nblocks = (pairs + blk - 1) / blk;
 }
 
+__global__ void subtract_local(const unsigned long long *__restrict__ src, const LocalSub sub, uint64_t total) {
+    for (uint64_t t = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; t < total;
+         t += (uint64_t)gridDim.x * blockDim.x) {
+        const uint64_t v = t / sub.n;
+        const unsigned long long c = src[v * sub.src_n + sub.block[t - v * sub.n]];
+        if (c) sub.dst[t] -= c;
+    }
+}
+
+// Takes the embeddings of the quotients of queries with far pairs off their
+// maps (far_quotients), which blocks and counts hold; done[k] is cleared where
+// query k is better, or has to be, enumerated itself.
+int subtract_quotients(asdm_graph *G, const std::vector<asdm_cs *> &cs, const std::vector<unsigned long long *> &blocks,
+                       std::vector<uint64_t> &counts, std::vector<char> &done, asdm_run_stats *agg) {
+    struct Job { size_t k; std::unique_ptr<asdm_cs> c; LocalSub sub; };
+    std::vector<Job> jobs;
+    for (size_t k = 0; k < cs.size(); ++k) {
+        std::vector<Quotient> quots;
+        if (!done[k] || tree_countable_conflicts(cs[k]->q)) continue;
+        if (counts[k] < kQuotientMaps || !far_quotients(*cs[k], quots)) {
+            done[k] = 0;
+            continue;
+        }
+        for (Quotient &x : quots) {
+            Job j{k, std::make_unique<asdm_cs>(), LocalSub{}};
+            j.c->g = G;
+            j.c->q = std::move(x.q);
+            j.sub.dst = blocks[k];
+            j.sub.n = cs[k]->q.n;
+            j.sub.src_n = j.c->q.n;
+            for (uint32_t u = 0; u < j.sub.n; ++u) j.sub.block[u] = (uint8_t)x.block[u];
+            jobs.push_back(std::move(j));
+        }
+    }
+    int rc = ASDM_OK;
+    for (size_t at = 0; at < jobs.size() && rc == ASDM_OK;) {
+        // up to 2 GiB of local-count blocks per launch
+        const size_t first = at;
+        uint64_t words = 0;
+        std::vector<asdm_cs *> group;
+        for (; at < jobs.size(); ++at) {
+            const uint64_t need = (uint64_t)G->d.n * jobs[at].sub.src_n;
+            if (!group.empty() && words + need > (1ull << 28)) break;
+            group.push_back(jobs[at].c.get());
+            words += need;
+        }
+        if ((rc = build_batch(group))) break;
+        std::vector<asdm_plan> plans(group.size());
+        std::vector<asdm_cs *> run;
+        std::vector<const asdm_plan *> rplans;
+        std::vector<LocalSub> subs;
+        std::vector<size_t> of;
+        for (size_t i = 0; i < group.size() && rc == ASDM_OK; ++i) {
+            if (!group[i]->nonempty) continue;
+            rc = build_plan(*group[i], nullptr, plans[i]);
+            run.push_back(group[i]);
+            rplans.push_back(&plans[i]);
+            subs.push_back(jobs[first + i].sub);
+            of.push_back(jobs[first + i].k);
+        }
+        if (rc != ASDM_OK || run.empty()) continue;
+        std::vector<uint64_t> c(run.size());
+        std::vector<int> st(run.size());
+        asdm_run_stats es{};
+        rc = run_batch_count(G, run, rplans, 0.0, 0, c.data(), st.data(), &es, nullptr, nullptr, 0.0,
+                             /*settled=*/true, nullptr, &subs);
+        for (size_t i = 0; i < run.size() && rc == ASDM_OK; ++i) {
+            if (st[i] != ASDM_OK) done[of[i]] = 0;
+            counts[of[i]] -= c[i];
+        }
+        if (agg) {
+            agg->intersections += es.intersections;
+            agg->list_bytes += es.list_bytes;
+            agg->tasks += es.tasks;
+            agg->busy_warp_ms += es.busy_warp_ms;
+            agg->idle_warp_ms += es.idle_warp_ms;
+        }
+    }
+    if (rc == ASDM_ERR_OOM) {  // no room for the quotients beside the rest
+        for (const Job &j : jobs) done[j.k] = 0;
+        clear_error();
+        rc = ASDM_OK;
+    }
+    return rc;
+}
+
 int run_plan(asdm_cs &cs, const asdm_plan &plan, const asdm_run_opts &opt, asdm_run_stats &st) {
     asdm_graph *G = cs.g;
     cudaStream_t s = G->stream;
@@ -1871,7 +1970,10 @@ int run_plan(asdm_cs &cs, const asdm_plan &plan, const asdm_run_opts &opt, asdm_
     HostFill fill;
     if (opt.local_counts && (mode & ASDM_MODE_LOCAL)) fill.start({{opt.local_counts, (uint64_t)G->d.n * n}});
     if (!cs.nonempty) return ASDM_OK;
-    if (mode == ASDM_MODE_LOCAL && opt.local_counts && plan.order.size() == n && tree_countable_conflicts(q)) {
+    std::vector<Quotient> quots;
+    // (runs with a time or count limit enumerate a query with far pairs itself)
+    if (mode == ASDM_MODE_LOCAL && opt.local_counts && plan.order.size() == n &&
+        (tree_countable_conflicts(q) || (!(opt.time_limit_s > 0) && !opt.count_limit && far_quotients(cs, quots)))) {
         // tree: counts and local counts from the tree program
         const uint64_t local_n = (uint64_t)G->d.n * n;
         unsigned long long *blk = nullptr;
@@ -1884,8 +1986,9 @@ int run_plan(asdm_cs &cs, const asdm_plan &plan, const asdm_run_opts &opt, asdm_
         std::vector<char> done;
         std::vector<unsigned long long *> blocks{blk};
         int trc = cudaMemsetAsync(blk, 0, local_n * sizeof(unsigned long long), s) == cudaSuccess
-                      ? tree_counts(G, {&cs}, tc, done, &blocks)
+                      ? tree_counts(G, {&cs}, tc, done, &blocks, /*near_only=*/true)
                       : fail(ASDM_ERR_CUDA, "local-count reset failed");
+        if (trc == ASDM_OK) trc = subtract_quotients(G, {&cs}, blocks, tc, done, &st);
         cudaEventRecord(t1, s);
         cudaEventSynchronize(t1);
         float tms = 0.f;
@@ -2115,17 +2218,21 @@ int run_plan(asdm_cs &cs, const asdm_plan &plan, const asdm_run_opts &opt, asdm_
 // queries with full[i] set (whole queries, not prefixes) take part.  live
 // holds the positions still open on entry and on return; counts and status of
 // the settled ones are written, their device time is added to agg->kernel_ms.
+// A run with a time or count limit (limited) enumerates trees with far pairs
+// themselves.
 int settle_queries(asdm_graph *G, const std::vector<asdm_cs *> &cs, const std::vector<char> &full,
                    std::vector<uint32_t> &live, uint64_t count_limit, uint64_t *counts, int *status,
-                   asdm_run_stats *agg, uint64_t *const *local_out, HostFill *fill) {
+                   asdm_run_stats *agg, uint64_t *const *local_out, HostFill *fill, bool limited) {
     cudaStream_t s = G->stream;
     const uint32_t Q = (uint32_t)cs.size();
     if (live.empty()) return ASDM_OK;
     float tree_ms = 0.f;
     if (local_out) {
         std::vector<uint32_t> tid;
+        std::vector<Quotient> quots;
         for (uint32_t i : live)
-            if (full[i] && tree_countable_conflicts(cs[i]->q)) tid.push_back(i);
+            if (full[i] && (tree_countable_conflicts(cs[i]->q) || (!limited && far_quotients(*cs[i], quots))))
+                tid.push_back(i);
         std::vector<char> settled(Q, 0);
         cudaEvent_t t0, t1;
         cudaEventCreate(&t0);
@@ -2155,8 +2262,9 @@ int settle_queries(asdm_graph *G, const std::vector<asdm_cs *> &cs, const std::v
             std::vector<uint64_t> tc;
             std::vector<char> done;
             trc = cudaMemsetAsync(blk, 0, words * sizeof(unsigned long long), s) == cudaSuccess
-                      ? tree_counts(G, tcs, tc, done, &blocks)
+                      ? tree_counts(G, tcs, tc, done, &blocks, /*near_only=*/true)
                       : fail(ASDM_ERR_CUDA, "local-count reset failed");
+            if (trc == ASDM_OK) trc = subtract_quotients(G, tcs, blocks, tc, done, agg);
             std::vector<LocalRead> reads;
             for (size_t k = 0; k < ids.size() && trc == ASDM_OK; ++k)
                 if (done[k] && local_out[ids[k]]) reads.push_back(LocalRead{cs[ids[k]], blocks[k], local_out[ids[k]]});
@@ -2269,7 +2377,8 @@ int settle_queries(asdm_graph *G, const std::vector<asdm_cs *> &cs, const std::v
 
 int run_batch_count(asdm_graph *G, const std::vector<asdm_cs *> &cs, const std::vector<const asdm_plan *> &plans,
                     double time_limit_s, uint64_t count_limit, uint64_t *counts, int *status, asdm_run_stats *agg,
-                    uint64_t *const *local_out, uint64_t *cycles, double query_time_s, bool settled, HostFill *fill) {
+                    uint64_t *const *local_out, uint64_t *cycles, double query_time_s, bool settled, HostFill *fill,
+                    const std::vector<LocalSub> *subs) {
     cudaStream_t s = G->stream;
     const uint32_t Q = (uint32_t)cs.size();
     std::vector<uint32_t> live;  // queries with a non-empty candidate space
@@ -2284,10 +2393,12 @@ int run_batch_count(asdm_graph *G, const std::vector<asdm_cs *> &cs, const std::
     if (!settled) {
         std::vector<char> full(Q, 0);
         for (uint32_t i = 0; i < Q; ++i) full[i] = plans[i]->order.size() == cs[i]->q.n;
-        ASDM_TRY(settle_queries(G, cs, full, live, count_limit, counts, status, agg, local_out, fill));
+        ASDM_TRY(settle_queries(G, cs, full, live, count_limit, counts, status, agg, local_out, fill,
+                                time_limit_s > 0 || query_time_s > 0 || count_limit));
         if (live.empty()) return ASDM_OK;
     }
     const uint32_t L = (uint32_t)live.size();
+    const bool local_mode = local_out != nullptr || subs != nullptr;
     // host images of all plans, then one upload
     std::vector<uint8_t> hp;
     struct Off { uint64_t lv, bk, cf; };
@@ -2334,7 +2445,7 @@ int run_batch_count(asdm_graph *G, const std::vector<asdm_cs *> &cs, const std::
         qd[li].nc = (uint32_t)cf.size();
         unsigned long long nt = 0;
         const uint32_t tm = tail_mode(plan);
-        const bool light = local_out == nullptr && n <= 4 && (tm == kTailChain || tm == kTailLeaf);
+        const bool light = !local_mode && n <= 4 && (tm == kTailChain || tm == kTailLeaf);
         root_blocks(c, plan, qd[li].pairs, qd[li].blk, nt, light ? light_blk : 1);
         task_pre[li + 1] = task_pre[li] + nt;
         maxn = std::max(maxn, n);
@@ -2352,7 +2463,6 @@ int run_batch_count(asdm_graph *G, const std::vector<asdm_cs *> &cs, const std::
     int rc = ASDM_OK;
     cudaEvent_t e0 = nullptr, e1 = nullptr;
     // local counts (LOCAL mode): one |Vg| x n block per live query
-    const bool local_mode = local_out != nullptr;
     std::vector<uint64_t> local_base(L + 1, 0);
     for (uint32_t li = 0; li < L; ++li)
         local_base[li + 1] = local_base[li] + (local_mode ? (uint64_t)G->d.n * cs[live[li]]->q.n : 0);
@@ -2534,7 +2644,17 @@ int run_batch_count(asdm_graph *G, const std::vector<asdm_cs *> &cs, const std::
             }
             rc = push_leaf_weights(tcs, tpl, lwv, blocks, G->num_sms, s);
         }
-        if (rc == ASDM_OK && local_mode) {
+        if (rc == ASDM_OK && subs) {
+            for (uint32_t li = 0; li < L; ++li) {
+                const LocalSub &sub = (*subs)[live[li]];
+                const uint64_t total = (uint64_t)G->d.n * sub.n;
+                const unsigned grid = (unsigned)std::min<uint64_t>((total + 255) / 256, (uint64_t)G->num_sms * 32);
+                subtract_local<<<grid, 256, 0, s>>>(d_local + local_base[li], sub, total);
+                ::asdm::count_launch();
+            }
+            if (cudaGetLastError() != cudaSuccess) rc = fail(ASDM_ERR_CUDA, "local-count update failed");
+        }
+        if (rc == ASDM_OK && local_out) {
             std::vector<LocalRead> reads;
             for (uint32_t li = 0; li < L; ++li)
                 if (local_out[live[li]]) reads.push_back(LocalRead{cs[live[li]], d_local + local_base[li], local_out[live[li]]});

@@ -224,6 +224,7 @@ int sorted_rows(const asdm_cs &cs, const RowLayout &lay, const unsigned long lon
                              lay.bits[u] == 32 ? 0xFFFFFFFFu : (1u << lay.bits[u]) - 1u, 0};
     RowField *d_fields = nullptr;
     uint32_t *d_out = nullptr;
+    unsigned long long *gathered = nullptr;
     const bool pairs = lay.words > 1;
     // on the device where its buffers fit and row numbers fit 32 bits
     SortBuffers b{s};
@@ -231,12 +232,14 @@ int sorted_rows(const asdm_cs &cs, const RowLayout &lay, const unsigned long lon
     if (device) {
         const uint64_t ntiles = (rows + kSortTile - 1) / kSortTile;
         device = ntiles <= 0x7FFFFFFFull && dalloc(&b.key[0], rows, s) == ASDM_OK && dalloc(&b.key[1], rows, s) == ASDM_OK &&
-                 (!pairs || (dalloc(&b.val[0], rows, s) == ASDM_OK && dalloc(&b.val[1], rows, s) == ASDM_OK)) &&
+                 (!pairs || (dalloc(&b.val[0], rows, s) == ASDM_OK && dalloc(&b.val[1], rows, s) == ASDM_OK &&
+                             dalloc(&gathered, rows, s) == ASDM_OK)) &&
                  dalloc(&b.hist, ntiles * kDigits, s) == ASDM_OK && dalloc(&b.pos, ntiles * kDigits + 1, s) == ASDM_OK &&
                  dalloc(&d_out, rows * n, s) == ASDM_OK;
         if (!device) {
             cudaGetLastError();
             clear_error();
+            dfree(gathered, s);
             dfree(d_out, s);
         }
     }
@@ -257,8 +260,6 @@ int sorted_rows(const asdm_cs &cs, const RowLayout &lay, const unsigned long lon
             } else {
                 iota_rows<<<grid_of(rows, G->num_sms), 256, 0, s>>>(b.val[0], rows);
                 ::asdm::count_launch();
-                unsigned long long *gathered = nullptr;
-                if ((rc = dalloc(&gathered, rows, s))) break;
                 for (uint32_t w = lay.words; w-- > 0 && rc == ASDM_OK;) {
                     gather_words<<<grid_of(rows, G->num_sms), 256, 0, s>>>(keys + (uint64_t)w * cap, b.val[at], rows,
                                                                           gathered);
@@ -266,7 +267,6 @@ int sorted_rows(const asdm_cs &cs, const RowLayout &lay, const unsigned long lon
                     const unsigned long long *unused = nullptr;
                     rc = radix_sort(b, gathered, rows, lay.word_bits[w], true, &at, &unused);
                 }
-                dfree(gathered, s);
                 if (rc != ASDM_OK) break;
             }
             unpack_rows<<<grid_of(rows * n, G->num_sms), 256, 0, s>>>(sorted, stride, pairs ? b.val[at] : nullptr, 0, rows,
@@ -302,6 +302,7 @@ int sorted_rows(const asdm_cs &cs, const RowLayout &lay, const unsigned long lon
         for (uint64_t r = 0; r < rows; ++r)
             std::memcpy(out + r * n, tmp.data() + perm[r] * n, n * sizeof(uint32_t));
     } while (false);
+    dfree(gathered, s);
     dfree(d_out, s);
     dfree(d_fields, s);
     cudaStreamSynchronize(s);  // the upload reads a host vector

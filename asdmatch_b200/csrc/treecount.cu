@@ -303,6 +303,7 @@ __global__ void tree_maps(const MapSeg *__restrict__ segs, uint32_t nseg, unsign
 
 constexpr size_t kMaxPartitions = 4096;  // partitions generated for one query
 constexpr size_t kMaxTerms = 64;         // terms counted for one query
+constexpr size_t kMaxNearBlock = 8;      // vertices of a block when only near pairs are held apart
 
 // One term of the inclusion-exclusion: a partition of the query vertices
 // into blocks, its quotient rooted at one block.
@@ -375,14 +376,48 @@ uint64_t term_cost(const BlockTree &t, const asdm_cs &c) {
     return cost;
 }
 
+// Whether u and w have a neighbour in common.
+bool near_pair(const QueryGraph &q, uint32_t u, uint32_t w) {
+    for (uint32_t e = q.off[u]; e < q.off[u + 1]; ++e)
+        if (q.slot(q.nbr[e], w) >= 0) return true;
+    return false;
+}
+
+// The coefficient of a block when only near pairs are held to be different:
+// the sum of (-1)^edges over the connected spanning subgraphs of the block's
+// near pairs (0 where they do not connect it; (-1)^(k-1) (k-1)! where every
+// pair of its k vertices is near).
+long long near_coef(const QueryGraph &q, const std::vector<uint32_t> &m) {
+    const uint32_t k = (uint32_t)m.size(), full = (1u << k) - 1;
+    std::vector<uint32_t> near(k, 0);
+    for (uint32_t a = 0; a < k; ++a)
+        for (uint32_t b = 0; b < k; ++b)
+            if (a != b && near_pair(q, m[a], m[b])) near[a] |= 1u << b;
+    auto apart = [&](uint32_t set) {  // no near pair in the set: the sum over all its subgraphs is 1, else 0
+        for (uint32_t a = 0; a < k; ++a)
+            if (set >> a & 1 && near[a] & set) return false;
+        return true;
+    };
+    std::vector<long long> c(full + 1, 0);
+    for (uint32_t set = 1; set <= full; ++set) {
+        const uint32_t low = set & (0u - set);
+        c[set] = apart(set) ? 1 : 0;
+        // less the subgraphs whose component at the lowest vertex is smaller
+        for (uint32_t sub = (set - 1) & set; sub; sub = (sub - 1) & set)
+            if (sub & low && apart(set ^ sub)) c[set] -= c[sub];
+    }
+    return c[full];
+}
+
 // Every term of a tree query's count; false when the query does not qualify
 // (not a tree, a quotient with a cycle, too many partitions).  With a built
 // candidate space each term is rooted where its program reads the fewest
 // list entries.  With classes (cls[u]: u's class, or kNone when u may take
 // any candidate), vertices of different classes never share a block: they
-// can never share a data vertex.
+// can never share a data vertex.  With near_only, only vertices two edges
+// apart are held to be different.
 bool block_trees(const QueryGraph &q, std::vector<BlockTree> &out, const asdm_cs *cs = nullptr,
-                 const std::vector<uint32_t> *cls = nullptr) {
+                 const std::vector<uint32_t> *cls = nullptr, bool near_only = false) {
     out.clear();
     if (q.n < 2 || q.off[q.n] != 2 * (q.n - 1)) return false;
     std::vector<uint32_t> block(q.n, kNone);
@@ -403,6 +438,13 @@ bool block_trees(const QueryGraph &q, std::vector<BlockTree> &out, const asdm_cs
                 for (size_t k = 2; k < m.size(); ++k) f *= (long long)k;
                 t.coef *= (m.size() % 2 == 0) ? -f : f;
                 t.identity = t.identity && m.size() == 1;
+            }
+            if (near_only) {
+                t.coef = 1;
+                for (const auto &m : members)
+                    if (m.size() > kMaxNearBlock) { ok = false; return; }
+                    else if (m.size() > 1) t.coef *= near_coef(q, m);
+                if (t.coef == 0) return;
             }
             if (!root_quotient(q, t) || out.size() >= kMaxTerms) { ok = false; return; }
             if (cs) {
@@ -458,7 +500,7 @@ namespace {
 // tree_counts for one chunk of queries (all of whose device state is
 // allocated at once).
 int tree_counts_chunk(asdm_graph *G, const std::vector<asdm_cs *> &cs, std::vector<uint64_t> &counts,
-                      std::vector<char> &done, const std::vector<unsigned long long *> *local) {
+                      std::vector<char> &done, const std::vector<unsigned long long *> *local, bool near_only) {
     cudaStream_t s = G->stream;
     const uint32_t Q = (uint32_t)cs.size();
     counts.assign(Q, 0);
@@ -485,7 +527,7 @@ int tree_counts_chunk(asdm_graph *G, const std::vector<asdm_cs *> &cs, std::vect
     };
     for (uint32_t qi = 0; qi < Q; ++qi) {
         const asdm_cs &c = *cs[qi];
-        if (!c.nonempty || !block_trees(c.q, trees[qi], &c)) continue;
+        if (!c.nonempty || !block_trees(c.q, trees[qi], &c, nullptr, near_only)) continue;
         woff[qi].resize(trees[qi].size());
         for (uint32_t ti = 0; ti < trees[qi].size(); ++ti) {
             const BlockTree &t = trees[qi][ti];
@@ -775,9 +817,9 @@ int tree_counts_chunk(asdm_graph *G, const std::vector<asdm_cs *> &cs, std::vect
 
 // Device words (weights and member maps) a query's tree program needs, or 0
 // when it does not qualify.
-uint64_t tree_words(const asdm_cs &c) {
+uint64_t tree_words(const asdm_cs &c, bool near_only) {
     std::vector<BlockTree> t;
-    if (!c.nonempty || !block_trees(c.q, t)) return 0;
+    if (!c.nonempty || !block_trees(c.q, t, nullptr, nullptr, near_only)) return 0;
     uint64_t w = 0;
     for (const BlockTree &bt : t)
         for (uint32_t b = 0; b < bt.nb; ++b) w += c.ncand[bt.rep[b]] * (1 + bt.members[b].size());
@@ -2509,12 +2551,87 @@ int overflow_bounds(asdm_graph *G, const std::vector<asdm_cs *> &cs, std::vector
     return rc;
 }
 
+// Trees with same-label vertices three or more edges apart (far pairs): with
+// only the near pairs (two edges apart) held to be different, every quotient
+// of the inclusion-exclusion is a tree, and the tree program counts the maps
+// that are injective around every vertex.  (The candidate space holds them
+// all: the degree and label-count filters ask for no more.)  Such a map is an
+// embedding of Q, or of exactly one quotient of Q by blocks of pairwise far
+// vertices, the one whose blocks are the map's fibres:
+//     embeddings(Q) = maps(Q) - sum over the quotients of embeddings(quotient),
+// and the same for local counts.  A quotient has a cycle through each merged
+// vertex, so it has far fewer embeddings than Q; they are enumerated.  False
+// where the query does not qualify, has many quotients, or has few maps by the
+// candidate edges' averages: then it is cheaper to enumerate Q itself.
+bool far_quotients(const asdm_cs &cs, std::vector<Quotient> &out) {
+    constexpr size_t kMaxQuotients = 4;
+    const QueryGraph &q = cs.q;
+    out.clear();
+    std::vector<BlockTree> t;
+    if (!cs.nonempty || q.n < 4 || q.off[q.n] != 2 * (q.n - 1)) return false;
+    double maps = 0.0;  // log2 of the homomorphisms, were all lists of an edge equally long
+    for (uint32_t u = 0; u < q.n; ++u) {
+        maps -= ((double)q.deg(u) - 1.0) * std::log2((double)cs.ncand[u]);
+        for (uint32_t e = q.off[u]; e < q.off[u + 1]; ++e)
+            if (u < q.nbr[e]) maps += std::log2((double)std::max<uint64_t>(cs.etotal[e], 1));
+    }
+    if (maps < std::log2((double)kQuotientEstimate) || !block_trees(q, t, nullptr, nullptr, true)) return false;
+    std::vector<uint32_t> block(q.n, kNone);
+    std::vector<std::vector<uint32_t>> members;
+    bool ok = true;
+    std::function<void(uint32_t)> place = [&](uint32_t u) {
+        if (!ok) return;
+        if (u == q.n) {
+            if (members.size() == q.n) return;  // Q itself
+            if (out.size() == kMaxQuotients) { ok = false; return; }
+            Quotient x;
+            x.block = block;
+            std::vector<uint32_t> off{0}, nbr, lab;
+            for (const auto &m : members) lab.push_back(q.lab[m[0]]);
+            for (const auto &m : members) {
+                std::vector<std::pair<uint32_t, uint32_t>> around;  // (label, block)
+                for (uint32_t v : m)
+                    for (uint32_t e = q.off[v]; e < q.off[v + 1]; ++e) {
+                        const uint32_t b = block[q.nbr[e]];
+                        around.emplace_back(lab[b], b);
+                    }
+                std::sort(around.begin(), around.end());
+                around.erase(std::unique(around.begin(), around.end()), around.end());
+                for (const auto &a : around) nbr.push_back(a.second);
+                off.push_back((uint32_t)nbr.size());
+            }
+            ok = make_query(off.data(), nbr.data(), lab.data(), (uint32_t)members.size(), x.q) == ASDM_OK;
+            out.push_back(std::move(x));
+            return;
+        }
+        for (uint32_t b = 0; b < members.size() && ok; ++b) {
+            bool far = q.lab[members[b][0]] == q.lab[u];
+            for (uint32_t w : members[b]) far = far && q.slot(u, w) < 0 && !near_pair(q, u, w);
+            if (!far) continue;
+            members[b].push_back(u);
+            block[u] = b;
+            place(u + 1);
+            members[b].pop_back();
+        }
+        if (!ok) return;
+        block[u] = (uint32_t)members.size();
+        members.push_back({u});
+        place(u + 1);
+        members.pop_back();
+    };
+    place(0);
+    if (!ok) out.clear();
+    return !out.empty();
+}
+
 // Counts every countable query of `cs` (non-empty candidate spaces on graph
 // G); done[i] = 1 and counts[i] set for the queries it settled.  With local
 // counts the top-down pass of every term follows.  Queries run in chunks of
-// at most kTreeChunkWords device words (one query alone may exceed it).
+// at most kTreeChunkWords device words (one query alone may exceed it).  With
+// near_only the result of a query with far pairs is its number of maps (see
+// far_quotients).
 int tree_counts(asdm_graph *G, const std::vector<asdm_cs *> &cs, std::vector<uint64_t> &counts,
-                std::vector<char> &done, const std::vector<unsigned long long *> *local) {
+                std::vector<char> &done, const std::vector<unsigned long long *> *local, bool near_only) {
     const size_t Q = cs.size();
     counts.assign(Q, 0);
     done.assign(Q, 0);
@@ -2525,7 +2642,7 @@ int tree_counts(asdm_graph *G, const std::vector<asdm_cs *> &cs, std::vector<uin
         std::vector<size_t> ids;
         uint64_t words = 0;
         for (; at < Q; ++at) {
-            const uint64_t w = tree_words(*cs[at]) * (local ? 3 : 1);  // list sums and the way up beside the weights
+            const uint64_t w = tree_words(*cs[at], near_only) * (local ? 3 : 1);  // list sums and the way up beside the weights
             if (!ids.empty() && words + w > kTreeChunkWords) break;
             words += w;
             part.push_back(cs[at]);
@@ -2534,7 +2651,7 @@ int tree_counts(asdm_graph *G, const std::vector<asdm_cs *> &cs, std::vector<uin
         }
         std::vector<uint64_t> pc;
         std::vector<char> pd;
-        const int rc = tree_counts_chunk(G, part, pc, pd, local ? &lpart : nullptr);
+        const int rc = tree_counts_chunk(G, part, pc, pd, local ? &lpart : nullptr, near_only);
         if (rc != ASDM_OK) {
             done.assign(Q, 0);
             return rc;

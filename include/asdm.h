@@ -110,8 +110,8 @@ int asdm_graph_free(asdm_graph *g);
 /* Knobs of the enumeration kernels, per data graph; chosen by the autotuner
  * (asdmatch_b200.autotune) by timing the caller's own batch.
  *   enum_min_blocks: register budget of the batched enumeration kernel, as
- *     resident 256-thread blocks per SM it must allow (1 = compiler's choice,
- *     up to 6); more blocks hide more load latency but spill registers.
+ *     resident 256-thread blocks per SM it must allow (1 or 2 = two, up to 6);
+ *     more blocks hide more load latency but spill registers.
  *   lane_leaf_max: the last query level is evaluated one partial match per
  *     lane (instead of one per warp) when its shortest list has at most this
  *     many entries (the merge / gallop split of the intersection).
@@ -123,9 +123,10 @@ typedef struct asdm_tuning {
     uint32_t planner;          /* ASDM_PLANNER_DP or ASDM_PLANNER_GREEDY */
     uint32_t root_block_min;   /* batches: fewest (level-0, level-1) pairs per root task of plans of at
                                   most 4 levels with a closed-form tail, 1..256 (default 64) */
-    uint32_t padded_cap_log2;  /* candidate edges of a group are filled into lists padded to their
-                                  label-run lengths when those total at most 2^this entries, else
-                                  counted first and filled exactly (20..34, default 33: 32 GiB) */
+    uint32_t padded_cap_log2;  /* candidate edges of a group are filled in one scan through a staging
+                                  buffer of their label-run lengths when those total at most 2^this
+                                  entries, else counted first and filled exactly (20..34, default 33:
+                                  32 GiB) */
     uint32_t merge_ratio;      /* intersection method: a list probed by a round of 32 driver entries
                                   is merged with them (32-entry windows) while its unread part is at
                                   most this many times the driver's unread part, else galloped
