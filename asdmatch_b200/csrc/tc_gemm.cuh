@@ -25,6 +25,8 @@
 #include <cuda_bf16.h>
 #include <cstdint>
 
+#include "mma_steps.h"
+
 namespace asdm {
 namespace tc {
 
@@ -160,7 +162,6 @@ __device__ void gemm_tile(const Operand &A, const Operand &B, int K, int c0, int
     asm volatile("tcgen05.fence::after_thread_sync;");
     const uint32_t tmem = *tmem_slot;
 
-    bool ok = true;
     const int nc = c1 - c0;
     const uint32_t idesc = idesc_bf16_f32();
     auto fetch = [&](int i) {  // chunk i of this CTA into its stage (an empty group past the end)
@@ -171,9 +172,7 @@ __device__ void gemm_tile(const Operand &A, const Operand &B, int K, int c0, int
         }
         asm volatile("cp.async.commit_group;");
     };
-#pragma unroll
-    for (int i = 0; i < kStages - 1; ++i) fetch(i);
-    for (int i = 0; i < nc && ok; ++i) {
+    auto issue = [&](int i) {
         asm volatile("cp.async.wait_group %0;" ::"n"(kStages - 2));  // chunk i has landed
         // make the generic-proxy smem writes visible to the tensor cores
         asm volatile("fence.proxy.async.shared::cta;");
@@ -196,15 +195,11 @@ __device__ void gemm_tile(const Operand &A, const Operand &B, int K, int c0, int
             asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
                 smem_u32(mbar + i % kStages)));
         }
-        // the next fetch goes into the stage that chunk i - 1 was read from
-        bool done = true;
-        if (i > 0) done = wait_phase(mbar + (i - 1) % kStages, (uint32_t)((i - 1) / kStages) & 1u);
-        ok = __syncthreads_and(done);
-        if (ok) fetch(i + kStages - 1);
-    }
+    };
+    // chunk i's commit covers the products of every chunk before it
+    auto wait = [&](int i) { return wait_phase(mbar + i % kStages, (uint32_t)(i / kStages) & 1u); };
+    const bool ok = run_chunks<kStages>(nc, fetch, issue, wait, [](bool x) { return __syncthreads_and(x) != 0; });
     asm volatile("cp.async.wait_all;");
-    // the last chunk's products (its commit covers all before it)
-    if (nc > 0) ok = __syncthreads_and(ok && wait_phase(mbar + (nc - 1) % kStages, (uint32_t)((nc - 1) / kStages) & 1u));
     asm volatile("tcgen05.fence::after_thread_sync;");
     if (ok) {
         const int row = m0 + warp * 32 + lane;
@@ -239,7 +234,7 @@ __device__ void gemm_tile(const Operand &A, const Operand &B, int K, int c0, int
             }
         }
     } else {
-        // a wait ran out (each was bounded; the last one covered every MMA in flight)
+        // a wait ran out; the products in flight had one more bounded wait (run_chunks)
         if (threadIdx.x == 0) atomicExch(err, 1u);
     }
     asm volatile("tcgen05.fence::before_thread_sync;");
