@@ -28,6 +28,7 @@
 #include <mutex>
 
 #include "cs.cuh"
+#include "idle_wait.h"
 #include "local.cuh"
 #include "rows.cuh"
 
@@ -78,13 +79,12 @@ enum : int {
 // took 44 ms instead of 30.)
 constexpr uint32_t kMailWords = 64;
 constexpr uint32_t kMaxWarps = 16384;         // bits of the idle bitmap
-enum : uint32_t { kMailEmpty = 0, kMailRecord = 1, kMailDone = 2 };
 static_assert((kCtrN - kCtrIdle) * 64 >= kMaxWarps && kMailWords >= 5 + 32, "donation layout");
-// An idle warp polls until it is handed a record, no warp is working any more
-// or the run's deadline passes; without a deadline it leaves after kIdleMaxNs
-// (the working warps then finish their own ranges, so no work is lost).
+// An idle warp polls until it is handed a record, no warp is working any more,
+// a stop flag is set or the run's deadline passes; without a deadline it leaves
+// after kIdleMaxNs (the working warps then finish their own ranges, so no work
+// is lost).
 constexpr uint64_t kIdleMaxNs = 3600ull * 1000000000ull;
-constexpr uint64_t kHandoffNs = 1000000000ull;  // longest wait for a record once claimed
 constexpr uint32_t kIdleSleepMaxNs = 512;       // poll back-off ceiling
 // A busy warp looks for idle warps every kDonateEvery steps of its search (a
 // step opens a node or fills a chunk: 1-2 thousand cycles), at the number of
@@ -1016,42 +1016,35 @@ struct Warp {
             for (uint32_t w = lane; w < nwarps; w += 32) atomicExch(a.mail + (uint64_t)w * kMailWords, kMailDone);
     }
 
+    // The waiting warp's side of idle_wait (lane 0).
+    struct IdleIo {
+        const EnumArgs &a;
+        uint32_t *mb, *word, bit, sleep;
+        __device__ bool ended() const { return *(volatile unsigned long long *)&a.ctr[kCtrDone] != 0; }
+        __device__ uint32_t mail() const { return *(volatile uint32_t *)mb; }
+        __device__ bool stopped() const { return *(volatile unsigned long long *)&a.ctr[kCtrFlags] & kStopFlags; }
+        __device__ uint64_t now() const { return globaltimer(); }
+        __device__ bool take_back() const { return atomicAnd(word, ~bit) & bit; }
+        __device__ void lost() const { atomicOr((unsigned int *)&a.ctr[kCtrFlags], kFlagTimeout); }
+        __device__ void nap() {
+            __nanosleep(sleep);
+            sleep = min(2 * sleep, kIdleSleepMaxNs);
+        }
+    };
+
     // Idle: waits for a record in this warp's mailbox.  False when no warp is
-    // working any more or the wait's time bound (the run's deadline, else
-    // kIdleMaxNs) has passed.
+    // working any more, the run is stopped or the wait's time bound (the run's
+    // deadline, else kIdleMaxNs) has passed.
     __device__ bool wait_work(uint64_t deadline) {
         bool got = false;
         if (lane == 0) {
-            uint32_t *mb = a.mail + (uint64_t)wid * kMailWords, *word = idle_bits() + (wid >> 5);
-            const uint32_t bit = 1u << (wid & 31u);
-            atomicExch(mb, kMailEmpty);
+            IdleIo io{a, a.mail + (uint64_t)wid * kMailWords, idle_bits() + (wid >> 5), 1u << (wid & 31u), 64};
+            atomicExch(io.mb, kMailEmpty);
             __threadfence();
-            atomicOr(word, bit);
+            atomicOr(io.word, io.bit);
             __threadfence();
             const uint64_t t0 = globaltimer();
-            uint64_t until = deadline ? deadline : t0 + kIdleMaxNs;
-            bool claimed = false;
-            uint32_t nap = 64;
-            // a run that ended before the mailbox was emptied shows in the end flag
-            bool wait = *(volatile unsigned long long *)&a.ctr[kCtrDone] == 0;
-            for (uint32_t it = 0; wait; ++it) {
-                const uint32_t f = *(volatile uint32_t *)mb;
-                if (f != kMailEmpty) {
-                    got = f == kMailRecord;
-                    break;
-                }
-                if ((it & 255u) == 255u && globaltimer() > until) {
-                    if (claimed) {  // a claimed warp's record did not come: cannot happen, not a count to trust
-                        atomicOr((unsigned int *)&a.ctr[kCtrFlags], kFlagTimeout);
-                        break;
-                    }
-                    if (atomicAnd(word, ~bit) & bit) break;
-                    claimed = true;  // a donor took the bit first: its record is on the way
-                    until = globaltimer() + kHandoffNs;
-                }
-                __nanosleep(nap);
-                nap = min(2 * nap, kIdleSleepMaxNs);
-            }
+            got = idle_wait(io, deadline ? deadline : t0 + kIdleMaxNs);
             idle_ns += globaltimer() - t0;
             __threadfence();
         }
