@@ -260,7 +260,7 @@ struct Warp {
     unsigned long long count = 0, inter = 0, elems = 0, tails_lane = 0, tails_warp = 0;
     bool overflow = false;
     uint32_t wid, nwarps;  // this warp's number in the grid, the grid's warps
-    unsigned long long working = ~0ull;  // working warps as of the last look
+    uint32_t working = ~0u;  // lane 0's copy counts: working warps as of the last look
     uint64_t idle_ns = 0;  // lane 0: time spent waiting for work
     uint64_t t_mark = 0;   // lane 0: when this warp's time was last charged to its query
     const unsigned long long *ps;        // kTailChain: prefix sums over the driver edge of level n-2
@@ -1302,9 +1302,12 @@ __device__ bool dfs(const EnumArgs &a, Warp<MODE, MULTI> &W, uint32_t lane, uint
     while (d >= base) {
         ++iter;
         if ((iter & (kDonateEvery - 1)) == 0) {
-            if (W.working < W.nwarps) W.try_donate(base, d);
-            // one load for the warp, used at the next look
-            asm volatile("ld.volatile.global.u64 %0, [%1];" : "=l"(W.working) : "l"(a.ctr + kCtrActive));
+            // one lane's copy decides: try_donate is the whole warp's, and
+            // lanes that had loaded at different times could hold different
+            // counts
+            if (__shfl_sync(kFull, W.working, 0) < W.nwarps) W.try_donate(base, d);
+            // used at the next look (the low half: there are at most kMaxWarps)
+            asm volatile("ld.volatile.global.u32 %0, [%1];" : "=r"(W.working) : "l"(a.ctr + kCtrActive));
         }
         if ((iter & (kCheckEvery - 1)) == 0 || W.count >= a.flush_at) {
             uint32_t st = 0;
