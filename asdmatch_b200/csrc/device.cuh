@@ -9,9 +9,13 @@
 
 #include "internal.h"
 
+// A failed allocation leaves its error with the runtime as well as returning
+// it, and the next launch check would find it there, in this call's fallback or
+// in the next call: whoever takes the error clears it (the context is intact).
 #define ASDM_CUDA(call)                                                                              \
     do {                                                                                             \
         cudaError_t e__ = (call);                                                                    \
+        if (e__ == cudaErrorMemoryAllocation) cudaGetLastError();                                    \
         if (e__ != cudaSuccess)                                                                      \
             return ::asdm::fail(e__ == cudaErrorMemoryAllocation ? ASDM_ERR_OOM : ASDM_ERR_CUDA,     \
                                 "%s: %s (%s:%d)", #call, cudaGetErrorString(e__), __FILE__, __LINE__); \
@@ -166,6 +170,7 @@ int dalloc(T **p, uint64_t count, cudaStream_t s) {
     *p = nullptr;
     if (count == 0) count = 1;
     cudaError_t e = cudaMallocAsync((void **)p, count * sizeof(T), s);
+    if (e == cudaErrorMemoryAllocation) cudaGetLastError();  // see ASDM_CUDA
     if (e != cudaSuccess)
         return fail(e == cudaErrorMemoryAllocation ? ASDM_ERR_OOM : ASDM_ERR_CUDA, "device allocation of %llu bytes: %s",
                     (unsigned long long)(count * sizeof(T)), cudaGetErrorString(e));
@@ -197,7 +202,10 @@ struct PinnedStage {
         if (cur == chunks.size()) {
             uint8_t *p = nullptr;
             const size_t sz = std::max<size_t>(need, 4u << 20);
-            if (cudaMallocHost((void **)&p, sz) != cudaSuccess) return nullptr;
+            if (cudaMallocHost((void **)&p, sz) != cudaSuccess) {
+                cudaGetLastError();
+                return nullptr;
+            }
             chunks.emplace_back(p, sz);
             off = 0;
         }

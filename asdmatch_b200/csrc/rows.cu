@@ -237,7 +237,6 @@ int sorted_rows(const asdm_cs &cs, const RowLayout &lay, const unsigned long lon
                  dalloc(&b.hist, ntiles * kDigits, s) == ASDM_OK && dalloc(&b.pos, ntiles * kDigits + 1, s) == ASDM_OK &&
                  dalloc(&d_out, rows * n, s) == ASDM_OK;
         if (!device) {
-            cudaGetLastError();
             clear_error();
             dfree(gathered, s);
             dfree(d_out, s);
