@@ -147,14 +147,27 @@ struct SortBuffers {
     uint32_t *val[2] = {nullptr, nullptr};
     uint32_t *hist = nullptr;
     uint64_t *pos = nullptr;
-    ~SortBuffers() {
+    unsigned long long *gathered = nullptr;
+    int alloc(uint64_t rows, bool pairs) {
+        const uint64_t ntiles = (rows + kSortTile - 1) / kSortTile;
+        for (int i = 0; i < 2; ++i) {
+            ASDM_TRY(dalloc(&key[i], rows, s));
+            if (pairs) ASDM_TRY(dalloc(&val[i], rows, s));
+        }
+        if (pairs) ASDM_TRY(dalloc(&gathered, rows, s));
+        ASDM_TRY(dalloc(&hist, ntiles * kDigits, s));
+        return dalloc(&pos, ntiles * kDigits + 1, s);
+    }
+    void release() {
         for (int i = 0; i < 2; ++i) {
             dfree(key[i], s);
             dfree(val[i], s);
         }
         dfree(hist, s);
         dfree(pos, s);
+        dfree(gathered, s);
     }
+    ~SortBuffers() { release(); }
 };
 
 // Sorts src (and, with values, val[*at]) by its low `bits` bits.  On return
@@ -212,6 +225,48 @@ RowLayout row_layout(const asdm_cs &cs) {
     return lay;
 }
 
+namespace {
+
+// The sorted rows in out, by way of the device's sort; ASDM_ERR_OOM where its
+// buffers do not fit (keys are left as they were).
+int device_sorted(const RowLayout &lay, const unsigned long long *keys, uint64_t cap, uint64_t rows,
+                  const RowField *d_fields, uint32_t n, int num_sms, cudaStream_t s, uint32_t *out) {
+    const bool pairs = lay.words > 1;
+    SortBuffers b{s};
+    ASDM_TRY(b.alloc(rows, pairs));
+    uint32_t *d_out = nullptr;
+    ASDM_TRY(dalloc(&d_out, rows * n, s));
+    const unsigned long long *sorted = keys;
+    uint64_t stride = cap;
+    int at = 0, rc = ASDM_OK;
+    if (!pairs) {
+        rc = radix_sort(b, keys, rows, lay.word_bits[0], false, &at, &sorted);
+        stride = rows;
+    } else {
+        iota_rows<<<grid_of(rows, num_sms), 256, 0, s>>>(b.val[0], rows);
+        ::asdm::count_launch();
+        for (uint32_t w = lay.words; w-- > 0 && rc == ASDM_OK;) {
+            gather_words<<<grid_of(rows, num_sms), 256, 0, s>>>(keys + (uint64_t)w * cap, b.val[at], rows, b.gathered);
+            ::asdm::count_launch();
+            const unsigned long long *unused = nullptr;
+            rc = radix_sort(b, b.gathered, rows, lay.word_bits[w], true, &at, &unused);
+        }
+    }
+    if (rc == ASDM_OK) {
+        unpack_rows<<<grid_of(rows * n, num_sms), 256, 0, s>>>(sorted, stride, pairs ? b.val[at] : nullptr, 0, rows,
+                                                               d_fields, n, d_out);
+        ::asdm::count_launch();
+        if (cudaGetLastError() != cudaSuccess ||
+            cudaMemcpyAsync(out, d_out, rows * n * sizeof(uint32_t), cudaMemcpyDeviceToHost, s) != cudaSuccess ||
+            cudaStreamSynchronize(s) != cudaSuccess)
+            rc = fail(ASDM_ERR_CUDA, "embedding readback failed");
+    }
+    dfree(d_out, s);
+    return rc;
+}
+
+}  // namespace
+
 int sorted_rows(const asdm_cs &cs, const RowLayout &lay, const unsigned long long *keys, uint64_t cap, uint64_t rows,
                 uint32_t *out) {
     if (rows == 0) return ASDM_OK;
@@ -224,24 +279,6 @@ int sorted_rows(const asdm_cs &cs, const RowLayout &lay, const unsigned long lon
                              lay.bits[u] == 32 ? 0xFFFFFFFFu : (1u << lay.bits[u]) - 1u, 0};
     RowField *d_fields = nullptr;
     uint32_t *d_out = nullptr;
-    unsigned long long *gathered = nullptr;
-    const bool pairs = lay.words > 1;
-    // on the device where its buffers fit and row numbers fit 32 bits
-    SortBuffers b{s};
-    bool device = rows >= kHostSortRows && (!pairs || rows < 0xFFFFFFFFull);
-    if (device) {
-        const uint64_t ntiles = (rows + kSortTile - 1) / kSortTile;
-        device = ntiles <= 0x7FFFFFFFull && dalloc(&b.key[0], rows, s) == ASDM_OK && dalloc(&b.key[1], rows, s) == ASDM_OK &&
-                 (!pairs || (dalloc(&b.val[0], rows, s) == ASDM_OK && dalloc(&b.val[1], rows, s) == ASDM_OK &&
-                             dalloc(&gathered, rows, s) == ASDM_OK)) &&
-                 dalloc(&b.hist, ntiles * kDigits, s) == ASDM_OK && dalloc(&b.pos, ntiles * kDigits + 1, s) == ASDM_OK &&
-                 dalloc(&d_out, rows * n, s) == ASDM_OK;
-        if (!device) {
-            clear_error();
-            dfree(gathered, s);
-            dfree(d_out, s);
-        }
-    }
     int rc = ASDM_OK;
     do {
         if ((rc = dalloc(&d_fields, n, s))) break;
@@ -249,38 +286,18 @@ int sorted_rows(const asdm_cs &cs, const RowLayout &lay, const unsigned long lon
             rc = fail(ASDM_ERR_CUDA, "row layout upload failed");
             break;
         }
-        if (device) {
-            const unsigned long long *sorted = keys;
-            uint64_t stride = cap;
-            int at = 0;
-            if (!pairs) {
-                if ((rc = radix_sort(b, keys, rows, lay.word_bits[0], false, &at, &sorted))) break;
-                stride = rows;
-            } else {
-                iota_rows<<<grid_of(rows, G->num_sms), 256, 0, s>>>(b.val[0], rows);
-                ::asdm::count_launch();
-                for (uint32_t w = lay.words; w-- > 0 && rc == ASDM_OK;) {
-                    gather_words<<<grid_of(rows, G->num_sms), 256, 0, s>>>(keys + (uint64_t)w * cap, b.val[at], rows,
-                                                                          gathered);
-                    ::asdm::count_launch();
-                    const unsigned long long *unused = nullptr;
-                    rc = radix_sort(b, gathered, rows, lay.word_bits[w], true, &at, &unused);
-                }
-                if (rc != ASDM_OK) break;
-            }
-            unpack_rows<<<grid_of(rows * n, G->num_sms), 256, 0, s>>>(sorted, stride, pairs ? b.val[at] : nullptr, 0, rows,
-                                                                     d_fields, n, d_out);
-            ::asdm::count_launch();
-            if (cudaGetLastError() != cudaSuccess ||
-                cudaMemcpyAsync(out, d_out, rows * n * sizeof(uint32_t), cudaMemcpyDeviceToHost, s) != cudaSuccess ||
-                cudaStreamSynchronize(s) != cudaSuccess)
-                rc = fail(ASDM_ERR_CUDA, "embedding readback failed");
-            break;
+        // on the device where its buffers fit, row numbers fit 32 bits and tiles a grid
+        if (rows >= kHostSortRows && (lay.words == 1 || rows < 0xFFFFFFFFull) && rows / kSortTile < 0x7FFFFFFFull) {
+            rc = device_sorted(lay, keys, cap, rows, d_fields, n, G->num_sms, s, out);
+            if (rc != ASDM_ERR_OOM) break;
         }
-        // unpacked in pieces of up to 64 MiB, sorted on the host
+        // unpacked in pieces of up to 64 MiB (smaller ones where those do not
+        // fit), sorted on the host
         std::vector<uint32_t> tmp(rows * n);
-        const uint64_t piece = std::min<uint64_t>(rows, std::max<uint64_t>(1, (16ull << 20) / n));
-        if ((rc = dalloc(&d_out, piece * n, s))) break;
+        uint64_t piece = std::min<uint64_t>(rows, std::max<uint64_t>(1, (16ull << 20) / n));
+        while ((rc = dalloc(&d_out, piece * n, s)) == ASDM_ERR_OOM && piece > 1) piece /= 2;
+        if (rc != ASDM_OK) break;
+        clear_error();  // of what did not fit
         for (uint64_t r = 0; r < rows && rc == ASDM_OK; r += piece) {
             const uint64_t m = std::min(piece, rows - r);
             unpack_rows<<<grid_of(m * n, G->num_sms), 256, 0, s>>>(keys, cap, nullptr, r, m, d_fields, n, d_out);
@@ -301,7 +318,6 @@ int sorted_rows(const asdm_cs &cs, const RowLayout &lay, const unsigned long lon
         for (uint64_t r = 0; r < rows; ++r)
             std::memcpy(out + r * n, tmp.data() + perm[r] * n, n * sizeof(uint32_t));
     } while (false);
-    dfree(gathered, s);
     dfree(d_out, s);
     dfree(d_fields, s);
     cudaStreamSynchronize(s);  // the upload reads a host vector

@@ -74,3 +74,15 @@ def test_quotients_of_a_batch_do_not_fit(far):
         counts, status, local = A.run_batch_local(dg, [edge, q])
     assert status.tolist() == [A.OK, A.OK] and counts.tolist() == [want.count, whole.count]
     assert np.array_equal(local[0], want.local_counts) and np.array_equal(local[1], whole.local_counts)
+
+# four million rows: keys 32 MB, the sort's two key buffers 64 MB and its output 48 MB
+@pytest.mark.parametrize("mb", [256, 128, 96, 64])
+def test_sort_does_not_fit(mb):
+    a, c = np.arange(2000), np.arange(2001, 4001)
+    edges = np.stack([np.concatenate([a, c]), np.full(4000, 2000)], 1)
+    dg = A.DeviceGraph(A.HostGraph.from_edges(4001, [0] * 2000 + [1] + [2] * 2000, edges))
+    q = A.HostGraph.from_edges(3, [0, 1, 2], [[0, 1], [1, 2]])
+    with contextlib.closing(dg), contextlib.closing(A.CandidateSpace(dg, q)) as cs:
+        with device_memory(mb):
+            rows = A.adaptive_share_join(cs, mode=A.MODE_EMBED, emb_capacity=4_000_000).embeddings
+    assert np.array_equal(rows, np.stack([np.repeat(a, 2000), np.full(4_000_000, 2000), np.tile(c, 2000)], 1))
