@@ -1971,17 +1971,19 @@ int run_plan(asdm_cs &cs, const asdm_plan &plan, const asdm_run_opts &opt, asdm_
     if (mode == ASDM_MODE_LOCAL && opt.local_counts && plan.order.size() == n &&
         (tree_countable_conflicts(q) || (!(opt.time_limit_s > 0) && !opt.count_limit && far_quotients(cs, quots)))) {
         // tree: counts and local counts from the tree program
+        // (enumerated below where the program's arrays do not fit)
         const uint64_t local_n = (uint64_t)G->d.n * n;
         unsigned long long *blk = nullptr;
-        ASDM_TRY(dalloc(&blk, local_n, s));
         cudaEvent_t t0, t1;
         cudaEventCreate(&t0);
         cudaEventCreate(&t1);
         cudaEventRecord(t0, s);
         std::vector<uint64_t> tc;
-        std::vector<char> done;
+        std::vector<char> done{0};
+        int trc = dalloc(&blk, local_n, s);
         std::vector<unsigned long long *> blocks{blk};
-        int trc = cudaMemsetAsync(blk, 0, local_n * sizeof(unsigned long long), s) == cudaSuccess
+        if (trc == ASDM_OK)
+            trc = cudaMemsetAsync(blk, 0, local_n * sizeof(unsigned long long), s) == cudaSuccess
                       ? tree_counts(G, {&cs}, tc, done, &blocks, /*near_only=*/true)
                       : fail(ASDM_ERR_CUDA, "local-count reset failed");
         if (trc == ASDM_OK) trc = subtract_quotients(G, {&cs}, blocks, tc, done, &st);
@@ -1994,8 +1996,12 @@ int run_plan(asdm_cs &cs, const asdm_plan &plan, const asdm_run_opts &opt, asdm_
         if (trc == ASDM_OK && done[0]) trc = read_locals(G, {LocalRead{&cs, blk, opt.local_counts}}, fill);
         dfree(blk, s);
         cudaStreamSynchronize(s);
-        if (trc != ASDM_OK) return trc;
-        if (done[0]) {
+        if (trc == ASDM_ERR_OOM) {
+            st = asdm_run_stats{};
+            clear_error();
+        } else if (trc != ASDM_OK) {
+            return trc;
+        } else if (done[0]) {
             st.count = tc[0];
             st.kernel_ms = tms;
             if (opt.count_limit && st.count > opt.count_limit) return fail(ASDM_ERR_LIMIT, "count limit reached");
@@ -2209,7 +2215,8 @@ int run_plan(asdm_cs &cs, const asdm_plan &plan, const asdm_run_opts &opt, asdm_
 // counts[i] / status[i] receive each query's result.
 // Queries settled without enumeration, before any plan is needed: tree
 // queries counted by the tree program (in LOCAL mode with their local counts,
-// a few queries at a time), then queries whose count
+// a few queries at a time; those for which it does not fit the device's memory
+// stay open), then queries whose count
 // a device lower bound shows to be at least 2^64 (ASDM_ERR_OVERFLOW).  Only
 // queries with full[i] set (whole queries, not prefixes) take part.  live
 // holds the positions still open on entry and on return; counts and status of
@@ -2248,7 +2255,7 @@ int settle_queries(asdm_graph *G, const std::vector<asdm_cs *> &cs, const std::v
                 words += need;
             }
             unsigned long long *blk = nullptr;
-            if ((trc = dalloc(&blk, words, s))) break;
+            trc = dalloc(&blk, words, s);
             std::vector<unsigned long long *> blocks;
             uint64_t o = 0;
             for (uint32_t i : ids) {
@@ -2257,9 +2264,10 @@ int settle_queries(asdm_graph *G, const std::vector<asdm_cs *> &cs, const std::v
             }
             std::vector<uint64_t> tc;
             std::vector<char> done;
-            trc = cudaMemsetAsync(blk, 0, words * sizeof(unsigned long long), s) == cudaSuccess
-                      ? tree_counts(G, tcs, tc, done, &blocks, /*near_only=*/true)
-                      : fail(ASDM_ERR_CUDA, "local-count reset failed");
+            if (trc == ASDM_OK)
+                trc = cudaMemsetAsync(blk, 0, words * sizeof(unsigned long long), s) == cudaSuccess
+                          ? tree_counts(G, tcs, tc, done, &blocks, /*near_only=*/true)
+                          : fail(ASDM_ERR_CUDA, "local-count reset failed");
             if (trc == ASDM_OK) trc = subtract_quotients(G, tcs, blocks, tc, done, agg);
             std::vector<LocalRead> reads;
             for (size_t k = 0; k < ids.size() && trc == ASDM_OK; ++k)
@@ -2273,8 +2281,12 @@ int settle_queries(asdm_graph *G, const std::vector<asdm_cs *> &cs, const std::v
                 if (count_limit && tc[k] > count_limit) status[i] = ASDM_ERR_LIMIT;
                 if (agg) agg->count += tc[k];
             }
-            if (cudaStreamSynchronize(s) != cudaSuccess && trc == ASDM_OK) trc = fail(ASDM_ERR_CUDA, "local-count readback failed");
+            if (cudaStreamSynchronize(s) != cudaSuccess) trc = fail(ASDM_ERR_CUDA, "local-count readback failed");
             dfree(blk, s);
+            if (trc == ASDM_ERR_OOM) {  // no room for the program's arrays: these queries stay open
+                trc = ASDM_OK;
+                clear_error();
+            }
         }
         cudaEventRecord(t1, s);
         cudaEventSynchronize(t1);

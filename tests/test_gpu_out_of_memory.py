@@ -75,6 +75,37 @@ def test_quotients_of_a_batch_do_not_fit(far):
     assert status.tolist() == [A.OK, A.OK] and counts.tolist() == [want.count, whole.count]
     assert np.array_equal(local[0], want.local_counts) and np.array_equal(local[1], whole.local_counts)
 
+@pytest.fixture(scope="module")
+def star():
+    """A centre with four leaves of one label: 15 terms, each with weights, list sums and ways up."""
+    rng = np.random.default_rng(3)
+    n = 400_000
+    e = np.unique(np.sort(rng.integers(0, n, (2_000_000, 2)), 1), axis=0)
+    dg = A.DeviceGraph(A.HostGraph.from_edges(n, rng.integers(0, 2, n), e[e[:, 0] != e[:, 1]]))
+    q = A.HostGraph.from_edges(5, [0, 1, 1, 1, 1], [[0, i] for i in range(1, 5)])
+    with contextlib.closing(dg), contextlib.closing(A.CandidateSpace(dg, q)) as cs:
+        yield dg, q, cs, A.adaptive_share_join(cs, mode=A.MODE_LOCAL)
+
+
+@pytest.mark.parametrize("mb", [64, 128])
+def test_tree_program_does_not_fit(star, mb):
+    dg, q, cs, whole = star
+    with device_memory(mb):
+        r = A.adaptive_share_join(cs, mode=A.MODE_LOCAL)
+    assert whole.list_bytes == 0 and r.list_bytes > 0  # enumerated
+    assert r.count == whole.count and np.array_equal(r.local_counts, whole.local_counts)
+
+
+def test_tree_program_of_a_batch_does_not_fit(star):
+    dg, q, cs, whole = star
+    edge = A.HostGraph.from_edges(2, [0, 1], [[0, 1]])
+    want = A.match(dg, edge, A.MODE_LOCAL)
+    with device_memory(192):
+        counts, status, local = A.run_batch_local(dg, [q, edge])
+    assert status.tolist() == [A.OK, A.OK] and counts.tolist() == [whole.count, want.count]
+    assert np.array_equal(local[0], whole.local_counts) and np.array_equal(local[1], want.local_counts)
+
+
 # four million rows: keys 32 MB, the sort's two key buffers 64 MB and its output 48 MB
 @pytest.mark.parametrize("mb", [256, 128, 96, 64])
 def test_sort_does_not_fit(mb):
