@@ -115,12 +115,20 @@ int read_locals(asdm_graph *G, const std::vector<LocalRead> &reads, HostFill &fi
     }
     GatherSeg *d_segs = nullptr;
     unsigned long long *d_val = nullptr;  // values, then vertices
+    const uint64_t words = total + (total + 1) / 2;
     std::vector<unsigned long long> back;
     int rc = ASDM_OK;
+    if (total && (rc = dalloc(&d_segs, segs.size(), s)) == ASDM_OK) rc = dalloc(&d_val, words, s);
+    if (rc == ASDM_ERR_OOM) {  // no room for the gathered entries: every matrix is copied whole
+        clear_error();
+        rc = ASDM_OK;
+        total = 0;
+        whole.clear();
+        for (const LocalRead &r : reads) whole.push_back(&r);
+    }
     do {
+        if (rc != ASDM_OK) break;
         if (total) {
-            const uint64_t words = total + (total + 1) / 2;
-            if ((rc = dalloc(&d_segs, segs.size(), s)) || (rc = dalloc(&d_val, words, s))) break;
             if (upload_async(G, d_segs, segs.data(), segs.size() * sizeof(GatherSeg)) != cudaSuccess) {
                 rc = fail(ASDM_ERR_CUDA, "local-count gather upload failed");
                 break;

@@ -106,6 +106,21 @@ def test_tree_program_of_a_batch_does_not_fit(star):
     assert np.array_equal(local[0], whole.local_counts) and np.array_equal(local[1], want.local_counts)
 
 
+def test_gathered_entries_do_not_fit():
+    k = 500_000  # disjoint cycles of six labels: a matrix of 144 MB, 36 MB of gathered entries
+    base = 6 * np.arange(k)[:, None]
+    edges = np.concatenate([base + [[i, (i + 1) % 6]] for i in range(6)])
+    dg = A.DeviceGraph(A.HostGraph.from_edges(6 * k, np.tile(np.arange(6), k), edges))
+    q = A.HostGraph.from_edges(6, range(6), [[i, (i + 1) % 6] for i in range(6)])
+    want = np.zeros((6 * k, 6), np.uint64)
+    want[np.arange(6 * k), np.tile(np.arange(6), k)] = 1
+    with contextlib.closing(dg), contextlib.closing(A.CandidateSpace(dg, q)) as cs:
+        for mb in (160, 512):
+            with device_memory(mb):
+                r = A.adaptive_share_join(cs, mode=A.MODE_LOCAL)
+            assert r.count == k and np.array_equal(r.local_counts, want)
+
+
 # four million rows: keys 32 MB, the sort's two key buffers 64 MB and its output 48 MB
 @pytest.mark.parametrize("mb", [256, 128, 96, 64])
 def test_sort_does_not_fit(mb):
