@@ -1507,8 +1507,12 @@ __device__ void warp_loop(const EnumArgs &a, Warp<MODE, MULTI> &W, uint32_t lane
     }
 }
 
+// LOCAL counts of one query keep three blocks per SM (79 registers), which the
+// compiler's own choice (80 or 107) comes to or not with small changes.  At two
+// blocks short searches are slower (0.65 to 0.69 ms, 0.59 to 0.66 ms) and long
+// ones faster (1.58 to 1.36 ms, 3.87 to 3.20 ms), counts on 3,112 vertices.
 template <uint32_t MODE>
-__global__ void __launch_bounds__(kThreads) enum_kernel(EnumArgs a) {
+__global__ void __launch_bounds__(kThreads, MODE == ASDM_MODE_LOCAL ? 3 : 1) enum_kernel(EnumArgs a) {
     extern __shared__ __align__(16) uint32_t sm[];
     DLevel *L = reinterpret_cast<DLevel *>(sm);
     DBack *B = reinterpret_cast<DBack *>(L + a.n);
