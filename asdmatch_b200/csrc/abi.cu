@@ -1,5 +1,7 @@
 // Remaining C-ABI entry points: batched set intersection (K4 as a standalone
 // primitive), the multi-query front end and the version string.
+#include <unistd.h>
+
 #include <algorithm>
 #include <atomic>
 #include <memory>
@@ -144,6 +146,32 @@ __global__ void __launch_bounds__(256) intersect_pack(uint32_t nsets, const uint
         if (c == chunk_pre[s] && lane == 0) out_count[s] = (uint32_t)(pos[chunk_pre[s + 1]] - base);
     }
 }
+
+// The calling thread's streams for work that belongs to no graph, one per
+// device: created on first use, destroyed when the thread ends.  They do not
+// synchronise with the legacy default stream, as cudaStreamPerThread does, so
+// the work runs beside whatever a program has there; creating and destroying a
+// stream in each call takes 110 us.
+struct ThreadStreams {
+    std::vector<std::pair<int, cudaStream_t>> all;
+    pid_t owner = getpid();
+    int get(int device, cudaStream_t *s) {
+        for (const auto &x : all)
+            if (x.first == device) {
+                *s = x.second;
+                return ASDM_OK;
+            }
+        all.reserve(all.size() + 1);
+        ASDM_CUDA(cudaStreamCreateWithFlags(s, cudaStreamNonBlocking));
+        all.emplace_back(device, *s);
+        return ASDM_OK;
+    }
+    ~ThreadStreams() {
+        if (getpid() != owner) return;  // a forked copy
+        for (const auto &x : all) cudaStreamDestroy(x.second);
+    }
+};
+thread_local ThreadStreams thread_streams;
 
 }  // namespace
 }  // namespace asdm
@@ -294,7 +322,8 @@ static int intersect_batch(const uint32_t *values, const uint64_t *list_off, uin
         if (chunks > 0xFFFFFFF0ull) return fail(ASDM_ERR_INVALID, "too many list entries");
     }
     idx.push_back((uint32_t)chunks);
-    cudaStream_t s = cudaStreamPerThread;  // the calling thread's own stream: nothing to create
+    cudaStream_t s = nullptr;
+    ASDM_TRY(thread_streams.get(dev, &s));
     uint32_t *d_vals = nullptr, *d_idx = nullptr, *d_out = nullptr, *d_cnt = nullptr, *d_stage = nullptr, *d_hits = nullptr;
     uint64_t *d_offs = nullptr, *d_pos = nullptr;
     int rc = ASDM_OK;
