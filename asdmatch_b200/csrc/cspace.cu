@@ -434,15 +434,15 @@ __device__ __forceinline__ uint32_t cand_index(const uint2 *cm, uint32_t r) {
     return (w.x & bit) ? w.y + (uint32_t)__popc(w.x & (bit - 1u)) : kNone;
 }
 
-// rstart (optional): each item's label-run start, its length in cnt (read
-// before cnt is overwritten with the count), both written by k3_bound.
+// Every item's list in one scan of its label run: its length in cnt, or (kFill)
+// its entries at elist + wpos[item].
 template <bool kFill>
 __global__ void __launch_bounds__(kBlock) k3_edges(DevGraph g, const EdgeDesc *__restrict__ edges,
                                                    const uint2 *__restrict__ cmem,
                                                    const uint64_t *__restrict__ item_base, uint32_t nedges,
                                                    uint32_t *__restrict__ cnt, const uint64_t *__restrict__ wpos,
-                                                   uint32_t *__restrict__ elist, unsigned long long *__restrict__ elems,
-                                                   const uint32_t *__restrict__ rstart) {
+                                                   uint32_t *__restrict__ elist,
+                                                   unsigned long long *__restrict__ elems) {
     const uint64_t total = item_base[nedges];
     const uint32_t lane = threadIdx.x & 31;
     const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
@@ -455,13 +455,8 @@ __global__ void __launch_bounds__(kBlock) k3_edges(DevGraph g, const EdgeDesc *_
         const uint32_t ei = warp_find_segment(item_base, nedges, base, item, pos < total, lane);
         if (pos < total) {
             const EdgeDesc d = edges[ei];
-            if (rstart) {
-                b = rstart[item];
-                e = b + cnt[item];
-            } else {
-                const uint32_t i = (uint32_t)(item - item_base[ei]);
-                if (i < d.ncand_u) label_run(g, d.cand_u[i], d.label_u2, b, e);
-            }
+            const uint32_t i = (uint32_t)(item - item_base[ei]);
+            if (i < d.ncand_u) label_run(g, d.cand_u[i], d.label_u2, b, e);
             cm = cmem + d.cmem;
         }
         scanned += e - b;
@@ -1201,29 +1196,34 @@ int build_batch(const std::vector<asdm_cs *> &group) {
         uint64_t bound = 0;
         uint32_t *rstart = nullptr;
         uint64_t *d_upos = nullptr;
-        // Small groups take the two-scan form too, whose four launches and no
-        // size readback are quicker than the chunked fill's eight and two
-        // (one 8-vertex query on 3,112 vertices: 490 -> 418 us a call).  Up to
-        // kListBound possible entries the lists get room for all of them; beyond,
-        // their exact length is read back first.  A group whose lists could pass
-        // the staging cap is not small: the cap decides about it below.
-        const uint64_t padded_cap = 1ull << G->tuning.padded_cap_log2;
-        const bool small = nitems <= kSmallItems && list_bound <= std::min(kSmallLists, padded_cap);
-        if (small) {
+        // The two scans; the lists get room for `room` entries, 0 for what the first scan counts.
+        auto count_then_fill = [&](uint64_t room) {
             ASDM_TRY(scr.alloc(&d_wpos, nitems + 1));
             k3_edges<false><<<egrid, kBlock, 0, s>>>(g, d_edges, cmem, d_ib, ne, arena->d_eoff, nullptr, nullptr,
-                                                    d_elems + 1, nullptr);
+                                                    d_elems + 1);
             ::asdm::count_launch();
+            ASDM_CUDA(cudaGetLastError());
             ASDM_TRY(scan_exclusive_u32(arena->d_eoff, d_wpos, nitems, true, s));
             ASDM_CUDA(cudaMemcpyAsync(&total, d_wpos + nitems, sizeof(uint64_t), cudaMemcpyDeviceToHost, s));
-            if (list_bound > kListBound) ASDM_CUDA(cudaStreamSynchronize(s));
-            ASDM_TRY(dalloc(&arena->d_elist, list_bound > kListBound ? total : list_bound, s));
-            k3_edges<true><<<egrid, kBlock, 0, s>>>(g, d_edges, cmem, d_ib, ne, nullptr, d_wpos, arena->d_elist,
-                                                    nullptr, nullptr);
+            if (!room) ASDM_CUDA(cudaStreamSynchronize(s));
+            ASDM_TRY(dalloc(&arena->d_elist, room ? room : total, s));
+            k3_edges<true><<<egrid, kBlock, 0, s>>>(g, d_edges, cmem, d_ib, ne, nullptr, d_wpos, arena->d_elist, nullptr);
             ::asdm::count_launch();
             k3_offsets<<<egrid, kBlock, 0, s>>>(d_ib, ne, d_wpos, arena->d_eoff, d_estart, d_bad);
             ::asdm::count_launch();
             ASDM_CUDA(cudaGetLastError());
+            return (int)ASDM_OK;
+        };
+        // Small groups take the two-scan form too, whose four launches and one
+        // readback are quicker than the chunked fill's eight and three
+        // (one 8-vertex query on 3,112 vertices: 490 -> 418 us a call).  Up to
+        // kListBound possible entries the lists get room for all of them.  A
+        // group whose lists could pass the staging cap is not small: the cap
+        // decides about it below.
+        const uint64_t padded_cap = 1ull << G->tuning.padded_cap_log2;
+        const bool small = nitems <= kSmallItems && list_bound <= std::min(kSmallLists, padded_cap);
+        if (small) {
+            ASDM_TRY(count_then_fill(list_bound > kListBound ? 0 : list_bound));
         } else {
             ASDM_TRY(scr.alloc(&rstart, nitems));
             ASDM_TRY(scr.alloc(&d_upos, nitems + 1));
@@ -1267,23 +1267,7 @@ int build_batch(const std::vector<asdm_cs *> &group) {
                 ASDM_CUDA(cudaGetLastError());
                 run_entries = bound;
             } else {
-                ASDM_TRY(scr.alloc(&d_wpos, nitems + 1));
-                k3_edges<false><<<egrid, kBlock, 0, s>>>(g, d_edges, cmem, d_ib, ne, arena->d_eoff, nullptr, nullptr,
-                                                        d_elems + 1, nullptr);
-                ::asdm::count_launch();
-                ASDM_CUDA(cudaGetLastError());
-                ASDM_TRY(scan_exclusive_u32(arena->d_eoff, d_wpos, nitems, true, s));
-                ASDM_CUDA(cudaMemcpyAsync(&total, d_wpos + nitems, sizeof(uint64_t), cudaMemcpyDeviceToHost, s));
-                ASDM_CUDA(cudaStreamSynchronize(s));
-                ASDM_TRY(dalloc(&arena->d_elist, total, s));
-                k3_edges<true><<<egrid, kBlock, 0, s>>>(g, d_edges, cmem, d_ib, ne, nullptr, d_wpos, arena->d_elist,
-                                                        nullptr, nullptr);
-                ::asdm::count_launch();
-                ASDM_CUDA(cudaGetLastError());
-                k3_offsets<<<grid_for(nitems, G->num_sms), kBlock, 0, s>>>(d_ib, ne, d_wpos, arena->d_eoff, d_estart,
-                                                                          d_bad);
-                ::asdm::count_launch();
-                ASDM_CUDA(cudaGetLastError());
+                ASDM_TRY(count_then_fill(0));
             }
         }
         uint32_t bad = 0;
@@ -1339,8 +1323,6 @@ int build_batch(const std::vector<asdm_cs *> &group) {
     return ASDM_OK;
 }
 
-namespace {
-}  // namespace
 }  // namespace asdm
 
 using namespace asdm;

@@ -1539,7 +1539,7 @@ __global__ void __launch_bounds__(kThreads, MODE == ASDM_MODE_LOCAL ? 3 : 1) enu
 // At least two blocks stay resident per SM (128 registers a thread) whatever
 // the tuning asks: at one, half of the warps that hide the loads are gone.
 template <int MINB, uint32_t MODE = ASDM_MODE_COUNT>
-__global__ void __launch_bounds__(kThreads, MINB < 2 ? 2 : MINB) enum_batch_kernel(EnumArgs a) {
+__global__ void __launch_bounds__(kThreads, MINB) enum_batch_kernel(EnumArgs a) {
     extern __shared__ __align__(16) uint32_t sm[];
     const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     uint32_t *wmem = sm + warp * warp_words(a.maxn, a.maxnb);
@@ -2563,17 +2563,16 @@ int run_batch_count(asdm_graph *G, const std::vector<asdm_cs *> &cs, const std::
         a.lane_leaf_max = G->tuning.lane_leaf_max;
         a.merge_ratio = G->tuning.merge_ratio;
         if (task_pre[L]) {
-            // register-budget variant chosen by the tuner (min blocks per SM)
-            void (*k)(EnumArgs) = enum_batch_kernel<1>;
+            // register-budget variant chosen by the tuner (min blocks per SM; 1 asks for the fewest, two)
+            void (*k)(EnumArgs) = enum_batch_kernel<2>;
             switch (G->tuning.enum_min_blocks) {
-                case 2: k = enum_batch_kernel<2>; break;
                 case 3: k = enum_batch_kernel<3>; break;
                 case 4: k = enum_batch_kernel<4>; break;
                 case 5: k = enum_batch_kernel<5>; break;
                 case 6: k = enum_batch_kernel<6>; break;
                 default: break;
             }
-            if (local_mode) k = enum_batch_kernel<1, ASDM_MODE_LOCAL>;
+            if (local_mode) k = enum_batch_kernel<2, ASDM_MODE_LOCAL>;
             if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) {
                 rc = fail(ASDM_ERR_CUDA, "shared-memory opt-in failed");
                 break;
