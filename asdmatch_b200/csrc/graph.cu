@@ -3,11 +3,37 @@
 // grouping (Graph::loadGraphFromTextFile, relation/graph.cpp:132-144) with a
 // counting sort, since it needs the id order preserved inside each label.
 #include <algorithm>
+#include <map>
 #include <memory>
+#include <mutex>
 
 #include "device.cuh"
 
 namespace asdm {
+
+// One pool per device, made on first use.  It keeps up to kKeptBytes that no
+// estimator uses (a new one then takes no time to get its buffers) and gives
+// the rest back.
+int kept_pool(int device, cudaMemPool_t *pool) {
+    constexpr uint64_t kKeptBytes = 256ull << 20;
+    static std::mutex mutex;
+    static std::map<int, cudaMemPool_t> pools;
+    std::lock_guard<std::mutex> lock(mutex);
+    const auto it = pools.find(device);
+    if (it != pools.end()) {
+        *pool = it->second;
+        return ASDM_OK;
+    }
+    cudaMemPoolProps props{};
+    props.allocType = cudaMemAllocationTypePinned;
+    props.location.type = cudaMemLocationTypeDevice;
+    props.location.id = device;
+    ASDM_CUDA(cudaMemPoolCreate(pool, &props));
+    uint64_t keep = kKeptBytes;
+    ASDM_CUDA(cudaMemPoolSetAttribute(*pool, cudaMemPoolAttrReleaseThreshold, &keep));
+    pools.emplace(device, *pool);
+    return ASDM_OK;
+}
 
 int device_setup(int *device, int *num_sms) {
     int count = 0;

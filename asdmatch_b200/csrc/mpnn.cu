@@ -280,21 +280,21 @@ int ensure_batch(asdm_estimator *e, int nodes, int graphs, uint64_t in_bytes) {
     if (in_bytes > e->cap_in) {
         dfree(e->in, s);
         e->cap_in = 0;
-        ASDM_TRY(dalloc(&e->in, in_bytes, s));
+        ASDM_TRY(dalloc_kept(&e->in, in_bytes, e->device, s));
         e->cap_in = in_bytes;
     }
     if (nodes <= e->cap_nodes && graphs <= e->cap_graphs) return ASDM_OK;
     free_batch(e);
     const int N = std::max(nodes, 1), G = std::max(graphs, 1);
-    ASDM_TRY(dalloc(&e->H, (uint64_t)(kLayers + 1) * N * kH, s));
-    ASDM_TRY(dalloc(&e->dH, (uint64_t)N * kH, s));
-    ASDM_TRY(dalloc(&e->dX, (uint64_t)N * kIn, s));
-    ASDM_TRY(dalloc(&e->gsum, (uint64_t)G * kH, s));
-    ASDM_TRY(dalloc(&e->y, G, s));
-    ASDM_TRY(dalloc(&e->dy, G, s));
-    ASDM_TRY(dalloc(&e->loss, 1, s));
-    ASDM_TRY(dalloc(&e->X, (uint64_t)kLayers * N * kIn, s));
-    ASDM_TRY(dalloc(&e->dZ, (uint64_t)N * kH, s));
+    ASDM_TRY(dalloc_kept(&e->H, (uint64_t)(kLayers + 1) * N * kH, e->device, s));
+    ASDM_TRY(dalloc_kept(&e->dH, (uint64_t)N * kH, e->device, s));
+    ASDM_TRY(dalloc_kept(&e->dX, (uint64_t)N * kIn, e->device, s));
+    ASDM_TRY(dalloc_kept(&e->gsum, (uint64_t)G * kH, e->device, s));
+    ASDM_TRY(dalloc_kept(&e->y, G, e->device, s));
+    ASDM_TRY(dalloc_kept(&e->dy, G, e->device, s));
+    ASDM_TRY(dalloc_kept(&e->loss, 1, e->device, s));
+    ASDM_TRY(dalloc_kept(&e->X, (uint64_t)kLayers * N * kIn, e->device, s));
+    ASDM_TRY(dalloc_kept(&e->dZ, (uint64_t)N * kH, e->device, s));
     e->cap_nodes = N;
     e->cap_graphs = G;
     return ASDM_OK;
@@ -400,13 +400,13 @@ extern "C" int asdm_est_create(uint32_t in_features, uint64_t seed, asdm_estimat
     e->in_features = in_features;
     e->nparam = 3 * asdm_estimator::kW + 3 * kH + kH + 1;
     cudaStream_t s = e->stream;
-    ASDM_TRY(dalloc(&e->p, e->nparam, s));
-    ASDM_TRY(dalloc(&e->g, e->nparam, s));
-    ASDM_TRY(dalloc(&e->m, e->nparam, s));
-    ASDM_TRY(dalloc(&e->v, e->nparam, s));
-    ASDM_TRY(dalloc(&e->wb, 3 * asdm_estimator::kW, s));
-    ASDM_TRY(dalloc(&e->err, 1, s));
-    ASDM_TRY(dalloc(&e->part, (uint64_t)asdm_estimator::kMaxSplits * asdm_estimator::kW, s));
+    ASDM_TRY(dalloc_kept(&e->p, e->nparam, e->device, s));
+    ASDM_TRY(dalloc_kept(&e->g, e->nparam, e->device, s));
+    ASDM_TRY(dalloc_kept(&e->m, e->nparam, e->device, s));
+    ASDM_TRY(dalloc_kept(&e->v, e->nparam, e->device, s));
+    ASDM_TRY(dalloc_kept(&e->wb, 3 * asdm_estimator::kW, e->device, s));
+    ASDM_TRY(dalloc_kept(&e->err, 1, e->device, s));
+    ASDM_TRY(dalloc_kept(&e->part, (uint64_t)asdm_estimator::kMaxSplits * asdm_estimator::kW, e->device, s));
     // Xavier-uniform weights from a seeded generator, zero biases
     std::vector<float> hp(e->nparam, 0.f);
     Rng rng(seed);
