@@ -638,7 +638,7 @@ def main():
                                            "same cap as a time limit)"},
                        batched_over_plain=plain_ms / ms,
                        decided_subset=decided,
-                       cs_build_roofline={"kernels": "K1-K3 (k1_filter, k2_pull, compaction, k3_bound/flat/pack)",
+                       cs_build_roofline={"kernels": "K1-K3 (k1_filter, k2_pull, compaction, k3_bound/fill/pack)",
                                           "bound": "hbm", "achieved": cs_achieved, "peak": peak, "unit": "GB/s",
                                           "frac": cs_achieved / peak, "algorithmic_bytes_per_step": cs_bytes,
                                           "device_ms_per_step": cs_ms, "traffic": traffic_cs},
