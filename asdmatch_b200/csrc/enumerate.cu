@@ -74,9 +74,9 @@ enum : int {
 // [flag, query, level s, lo, hi, idx[0..s-1]] into its mailbox.  Polls touch
 // only the poller's own line.  (A shared ring that every idle warp polled put
 // thousands of polls a microsecond on the line its head, tail and counters
-// share, and every handoff's atomics queued behind them: with chunk survivors
-// donated through it, the 64-query batch of 6 to 8 vertices on 3,112 vertices
-// took 44 ms instead of 30.)
+// share, and every handoff's atomics queued behind them.  The 64-query batch of
+// 6 to 8 vertices on 3,112 vertices took 73 ms with the ring, 16 ms with
+// mailboxes and chunk survivors given away too.)
 constexpr uint32_t kMailWords = 64;
 constexpr uint32_t kMaxWarps = 16384;         // bits of the idle bitmap
 static_assert((kCtrN - kCtrIdle) * 64 >= kMaxWarps && kMailWords >= 5 + 32, "donation layout");
